@@ -396,6 +396,9 @@ class CellList {
   const double* bbox(int s) const { return host_bbox_.data() + 6 * size_t(s); }
 
  private:
+  template <bool kTensor>
+  mf_status correction_at(const float4* tpos4, int64_t nt, const float4* pos4, const float4* mom4, float4* corr,
+                          cudaStream_t st) const;
   DevBuf grids_, bbox_, cell_start_, cursor_, perm_, perm_tmp_, cell_of_;
   DevBuf scan_tiles_;  // tile sums / offsets of the cell-count scan
   DevBuf skip_field_, skip_force_;  // per scene: 1 = not on the packed path

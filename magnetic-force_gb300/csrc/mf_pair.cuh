@@ -387,60 +387,6 @@ __device__ __forceinline__ void force_pair_sel(float dx, float dy, float dz, flo
   f[2] += dz * w + mz * u + sz * v;
 }
 
-// Correction of one near field pair (r^2 < near2): exact minus clamped,
-// accumulated as s1 (d (d.m) dalpha) and s2 (m dbeta) like the packed loop.
-__device__ __forceinline__ void field_near_correction(float dx, float dy, float dz, float mx, float my, float mz,
-                                                      const PairConsts<float>& pc, float alpha_c, float beta_c,
-                                                      float* s1, float* s2) {
-  const float r2 = dx * dx + dy * dy + dz * dz;
-  float alpha, beta;
-  field_near_coeffs<float>(r2, pc, alpha, beta);
-  const float da = alpha - alpha_c, db = beta - beta_c;
-  const float t = (dx * mx + dy * my + dz * mz) * da;
-  s1[0] += dx * t;
-  s1[1] += dy * t;
-  s1[2] += dz * t;
-  s2[0] += mx * db;
-  s2[1] += my * db;
-  s2[2] += mz * db;
-}
-
-// Correction of one near force pair (r^2 <= near2), contracted with m.
-// Tensor correction of one near pair (r^2 <= near2): exact minus clamped,
-// the 6 entries (xx, yy, zz, xy, xz, yz) of T / K.
-__device__ __forceinline__ void tensor_near_correction(float dx, float dy, float dz, float sx, float sy, float sz,
-                                                       const PairConsts<float>& pc, float P_c, float Q_c, float* t) {
-  const float r2 = dx * dx + dy * dy + dz * dz;
-  float P, Q;
-  force_near_coeffs<float>(r2, pc, P, Q);
-  const float dP = P - P_c, dQ = Q - Q_c;
-  const float ds = dx * sx + dy * sy + dz * sz;
-  const float pd = dP * ds, qd = dQ * ds;
-  const float ax = dP * sx, ay = dP * sy, az = dP * sz;
-  t[0] += pd + 2.f * ax * dx + qd * dx * dx;
-  t[1] += pd + 2.f * ay * dy + qd * dy * dy;
-  t[2] += pd + 2.f * az * dz + qd * dz * dz;
-  t[3] += ax * dy + ay * dx + qd * dx * dy;
-  t[4] += ax * dz + az * dx + qd * dx * dz;
-  t[5] += ay * dz + az * dy + qd * dy * dz;
-}
-
-__device__ __forceinline__ void force_near_correction(float dx, float dy, float dz, float sx, float sy, float sz,
-                                                      float mx, float my, float mz, const PairConsts<float>& pc,
-                                                      float P_c, float Q_c, float* f) {
-  const float r2 = dx * dx + dy * dy + dz * dz;
-  float P, Q;
-  force_near_coeffs<float>(r2, pc, P, Q);
-  const float dP = P - P_c, dQ = Q - Q_c;
-  const float ds = dx * sx + dy * sy + dz * sz;
-  const float dm = dx * mx + dy * my + dz * mz;
-  const float sm = sx * mx + sy * my + sz * mz;
-  const float u = dP * ds, v = dP * dm, w = dP * sm + dQ * ds * dm;
-  f[0] += dx * w + mx * u + sx * v;
-  f[1] += dy * w + my * u + sy * v;
-  f[2] += dz * w + mz * u + sz * v;
-}
-
 // One tensor pair (6 unique entries xx, yy, zz, xy, xz, yz): t += T(d, s) / K.
 template <class Real>
 __device__ __forceinline__ void tensor_pair(Real dx, Real dy, Real dz, Real sx, Real sy, Real sz,
