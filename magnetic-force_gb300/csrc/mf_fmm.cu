@@ -53,6 +53,21 @@ __host__ __device__ constexpr int gidx(int x, int y, int z) {
   return ncoef(x + y + z - 1) + (y + z) * (y + z + 1) / 2 + z;
 }
 
+// 1/|d| is harmonic, so D_(x, y, z + 2) = -D_(x + 2, y, z) - D_(x, y + 2, z):
+// the translation works on the multi-indices with z <= 1 only, 2 n + 1 of a
+// degree n instead of (n + 1)(n + 2)/2 (k_fmm_reduce, k_fmm_m2l, k_fmm_l2l).
+__host__ __device__ constexpr int nharm(int q) { return (q + 1) * (q + 1) - 1; }  // degrees 1..q
+__host__ __device__ constexpr int hidx(int x, int y, int z) {  // z <= 1
+  return nharm(x + y + z - 1) + (z == 0 ? y : x + y + 2 + y);
+}
+// Derivatives D_gamma with gamma_z <= 2 (3 n of a degree n >= 1), in rows of ndtab floats.
+__host__ __device__ constexpr int dofs(int n) { return n <= 0 ? 0 : 1 + 3 * n * (n - 1) / 2; }
+__host__ __device__ constexpr int didx(int x, int y, int z) {
+  const int n = x + y + z;
+  return dofs(n) + (z == 0 ? y : z == 1 ? n + 1 + y : 2 * n + 1 + y);
+}
+__host__ __device__ constexpr int ndtab(int q) { return (dofs(q + 2) + 3) / 4 * 4; }  // degrees 0..q + 1, whole float4
+
 // Multi-index table up to degree kMaxDegree + 1.
 __constant__ char4 c_mi[ncoef(kMaxDegree + 1)];
 // 1-D translation factors: c_shift[c][j] = ((c - 1/2) / 2)^j / j!, the child
@@ -336,35 +351,97 @@ __global__ void k_fmm_m2m(FmmLevel lc, FmmLevel lp, const int32_t* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// M2L:  L_beta += sum_alpha M_alpha D_(alpha + beta)(d),  |alpha| + |beta| <= Q + 1,
-// D_gamma(d) = d^gamma (1/|d|) at the box-centre offset d in box units.  The
-// sum is an unrolled program over compile-time (gamma, alpha, beta) triples,
-// gamma-major so each D value is loaded once; beta degrees BLO..BHI per
-// variant (two variants split the largest degrees so the multipole and the
-// accumulators both stay in registers).
+// Multipoles onto the indices with z <= 1 (every level from 2 on): with
+// D_(a, b, z + 2 j) = (-1)^j sum_i C(j, i) D_(a + 2 i, b + 2 (j - i), z),
+//   M'_(x, y, z) = sum_j (-1)^j sum_i C(j, i) M_(x - 2 i, y - 2 (j - i), z + 2 j),
+// the same potential outside the box, degree by degree.  One thread per
+// (coefficient, box); blockIdx.y is the level.
 // ---------------------------------------------------------------------------
-template <int Q, int BLO, int BHI>
+struct FmmLevels {
+  FmmLevel lv[kMaxLevel + 1];
+};
+__device__ __forceinline__ float binom_f(int j, int i) {  // j <= 5
+  float c = 1.f;
+  for (int k = 0; k < i; ++k) c = c * float(j - k) / float(k + 1);
+  return c;
+}
+
+template <int Q>
+__global__ void k_fmm_reduce(const FmmLevels lvs, int l0, const float* __restrict__ M, float* __restrict__ H,
+                             const double* __restrict__ done) {
+  constexpr int NC = ncoef(Q) - 1, NH = nharm(Q);
+  if (done && *done != 0.0) return;
+  const FmmLevel& lv = lvs.lv[l0 + blockIdx.y];
+  const float* m = M + lv.box_off * NC;
+  float* h = H + lv.box_off * NH;
+  for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < int64_t(NH) * lv.nbox;
+       t += int64_t(gridDim.x) * blockDim.x) {
+    const int k = int(t / lv.nbox);
+    const int64_t b = t % lv.nbox;
+    // k -> (x, y, z) of degree n: nharm(n - 1) <= k < nharm(n)
+    int n = 1;
+    while (k >= nharm(n)) ++n;
+    const int w = k - nharm(n - 1);
+    const int z = w <= n ? 0 : 1, y = w <= n ? w : w - n - 1, x = n - z - y;
+    float v = 0.f;
+    for (int j = 0; 2 * j <= x + y; ++j) {
+      float s = 0.f;
+      for (int i = 0; i <= j; ++i) {
+        const int a = x - 2 * i, c = y - 2 * (j - i);
+        if (a >= 0 && c >= 0) s += binom_f(j, i) * m[int64_t(gidx(a, c, z + 2 * j) - 1) * lv.nbox + b];
+      }
+      v += (j & 1) ? -s : s;
+    }
+    h[int64_t(k) * lv.nbox + b] = v;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// M2L:  L_beta += sum_alpha M'_alpha D_(alpha + beta)(d),  |alpha| + |beta| <= Q + 1,
+// D_gamma(d) = d^gamma (1/|d|) at the box-centre offset d in box units, over
+// the alpha and beta with z <= 1.  The locals with beta_z >= 2 follow from
+// these (L_beta are derivatives of a harmonic potential too, and the
+// truncation keeps whole degrees), so the result is the full sum's, at
+// sum (2|alpha| + 1)(2|beta| + 1) FMAs instead of one per full index pair:
+// 1,204 against 2,674 at Q = 7, 2,388 against ~6,500 for the force at Q = 9,
+// and 63 / 80 multipole loads instead of 119 / 219 (several times over: the
+// full sum needed two to four launches, each for a range of local degrees, to
+// keep the multipole and the accumulators in registers).  The sum is an
+// unrolled program over compile-time (gamma, alpha, beta) triples, gamma-major
+// so each D value is read once (four per load); local degrees BLO..Q.
+// Measured per step at 1,048,576 particles (one field product at Q = 7, one
+// force product at Q = 9): 13.6 ms for the full sum, 4.2 here (1.1 + 3.0; 168
+// and 249 registers).  Two launches split by local degree: 1.4 + 2.9 ms.
+// The kernel is bound by lanes without work: at the force's aperture about
+// half of the (target, list offset) pairs have no source box.
+// ---------------------------------------------------------------------------
+template <int Q, int BLO>
 struct M2LPlan {
   static constexpr int AMAX = (Q < Q + 1 - BLO) ? Q : Q + 1 - BLO;
-  static constexpr int NA = ncoef(AMAX) - 1;
-  static constexpr int BOFF = ncoef(BLO - 1);
-  static constexpr int NB = ncoef(BHI) - ncoef(BLO - 1);
+  static constexpr int NA = nharm(AMAX);
+  static constexpr int BOFF = nharm(BLO - 1);
+  static constexpr int NB = nharm(Q) - nharm(BLO - 1);
   struct Ent {
-    int16_t g, a, b, first;
+    int16_t g, a, b, first;  // first: this entry's gamma opens a new float4 of the row
   };
-  static constexpr int count() {
-    int k = 0;
+  template <class F>
+  static constexpr void walk(F&& f) {
     for (int g = BLO + 1; g <= Q + 1; ++g)
-      for (int s = 0; s <= g; ++s)
-        for (int gz = 0; gz <= s; ++gz) {
-          const int gy = s - gz, gx = g - s;
+      for (int gz = 0; gz <= 2 && gz <= g; ++gz)
+        for (int gy = 0; gy <= g - gz; ++gy) {
+          const int gx = g - gz - gy;
           for (int ax = 0; ax <= gx; ++ax)
             for (int ay = 0; ay <= gy; ++ay)
               for (int az = 0; az <= gz; ++az) {
                 const int a = ax + ay + az, b = g - a;
-                if (a >= 1 && a <= AMAX && b >= BLO && b <= BHI) ++k;
+                if (az > 1 || gz - az > 1 || a < 1 || a > AMAX || b < BLO || b > Q) continue;
+                f(didx(gx, gy, gz), hidx(ax, ay, az), hidx(gx - ax, gy - ay, gz - az) - BOFF);
               }
         }
+  }
+  static constexpr int count() {
+    int k = 0;
+    walk([&](int, int, int) { ++k; });
     return k;
   }
   static constexpr int K = count();
@@ -373,26 +450,15 @@ struct M2LPlan {
   };
   static constexpr Tab make() {
     Tab t{};
-    int k = 0;
-    for (int g = BLO + 1; g <= Q + 1; ++g)
-      for (int s = 0; s <= g; ++s)
-        for (int gz = 0; gz <= s; ++gz) {
-          const int gy = s - gz, gx = g - s;
-          bool first = true;
-          for (int ax = 0; ax <= gx; ++ax)
-            for (int ay = 0; ay <= gy; ++ay)
-              for (int az = 0; az <= gz; ++az) {
-                const int a = ax + ay + az, b = g - a;
-                if (a >= 1 && a <= AMAX && b >= BLO && b <= BHI) {
-                  t.e[k].g = int16_t(gidx(gx, gy, gz));
-                  t.e[k].a = int16_t(gidx(ax, ay, az) - 1);
-                  t.e[k].b = int16_t(gidx(gx - ax, gy - ay, gz - az) - BOFF);
-                  t.e[k].first = int16_t(first ? 1 : 0);
-                  first = false;
-                  ++k;
-                }
-              }
-        }
+    int k = 0, quad = -1;
+    walk([&](int g, int a, int b) {
+      t.e[k].g = int16_t(g);
+      t.e[k].a = int16_t(a);
+      t.e[k].b = int16_t(b);
+      t.e[k].first = int16_t(g / 4 != quad ? 1 : 0);
+      quad = g / 4;
+      ++k;
+    });
     return t;
   }
   static constexpr Tab tab = make();
@@ -403,16 +469,18 @@ struct M2LPlan {
 };
 
 template <class Pl, int I>
-__device__ __forceinline__ void m2l_step(float* acc, const float* M, const float* __restrict__ dt, float& dg) {
+__device__ __forceinline__ void m2l_step(float* acc, const float* M, const float4* __restrict__ dt, float4& dg) {
   using E = typename Pl::template At<I>;
-  if constexpr (E::first != 0) dg = __ldg(dt + E::g);
-  acc[E::b] = fmaf(M[E::a], dg, acc[E::b]);
+  if constexpr (E::first != 0) dg = __ldg(dt + E::g / 4);
+  constexpr int c = E::g % 4;
+  const float d = c == 0 ? dg.x : c == 1 ? dg.y : c == 2 ? dg.z : dg.w;
+  acc[E::b] = fmaf(M[E::a], d, acc[E::b]);
 }
 
 template <class Pl, int... Is>
-__device__ __forceinline__ void m2l_apply(float* acc, const float* M, const float* __restrict__ dt,
+__device__ __forceinline__ void m2l_apply(float* acc, const float* M, const float4* __restrict__ dt,
                                           std::integer_sequence<int, Is...>) {
-  float dg = 0.f;
+  float4 dg = make_float4(0.f, 0.f, 0.f, 0.f);
   (m2l_step<Pl, Is>(acc, M, dt, dg), ...);
 }
 
@@ -420,10 +488,10 @@ struct M2LArgs {
   FmmLevel lv;
   const int32_t* occ;   // sources per box
   const int32_t* tocc;  // targets per box
-  const float* M;     // this level's multipoles (NC rows of nbox)
-  float* Lp;          // [chunks][NC][nbox] partial locals
+  const float* M;     // this level's multipoles with z <= 1 (NH rows of nbox)
+  float* Lp;          // [chunks][NH][nbox] partial locals with z <= 1
   const int4* list;   // (dx, dy, dz, row of dtab)
-  const float* dtab;  // [rows][ncoef(Q + 1)]
+  const float4* dtab; // [rows][ndtab(Q) / 4]
   int64_t list_off[8];
   int32_t list_cnt[8];
   int32_t chunks;
@@ -434,11 +502,10 @@ struct M2LArgs {
 
 // One thread per (list chunk, target box); the warps of a block share the
 // chunk and the target parity class, so they walk the same offsets.
-template <int Q, int BLO, int BHI>
+template <int Q, int BLO>
 __global__ void __launch_bounds__(128) k_fmm_m2l(const M2LArgs p) {
-  using Pl = M2LPlan<Q, BLO, BHI>;
-  constexpr int NC = ncoef(Q) - 1;
-  constexpr int NG = ncoef(Q + 1);
+  using Pl = M2LPlan<Q, BLO>;
+  constexpr int NH = nharm(Q);
   if (p.done && *p.done != 0.0) return;
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t per = p.per_class;
@@ -470,23 +537,25 @@ __global__ void __launch_bounds__(128) k_fmm_m2l(const M2LArgs p) {
     float M[Pl::NA];
 #pragma unroll
     for (int q = 0; q < Pl::NA; ++q) M[q] = __ldg(p.M + int64_t(q) * lv.nbox + sb);
-    m2l_apply<Pl>(acc, M, p.dtab + int64_t(d.w) * NG, std::make_integer_sequence<int, Pl::K>{});
+    m2l_apply<Pl>(acc, M, p.dtab + int64_t(d.w) * (ndtab(Q) / 4), std::make_integer_sequence<int, Pl::K>{});
   }
-  float* out = p.Lp + int64_t(ch) * NC * lv.nbox;
+  float* out = p.Lp + int64_t(ch) * NH * lv.nbox;
 #pragma unroll
-  for (int q = 0; q < Pl::NB; ++q) out[int64_t(Pl::BOFF - 1 + q) * lv.nbox + tb] = acc[q];
+  for (int q = 0; q < Pl::NB; ++q) out[int64_t(Pl::BOFF + q) * lv.nbox + tb] = acc[q];
 }
 
 // Locals of a level: the M2L partials plus the parent's locals shifted to the
 // child centre,  L^c_beta += 2^(-2-|beta|) sum_delta L^p_(beta+delta) v_c^delta / delta!.
-// `occ` counts targets: boxes without targets need no locals.
+// `occ` counts targets: boxes without targets need no locals.  The partials
+// hold the locals with z <= 1; L_(x, y, z + 2 j) = (-1)^j sum_i C(j, i)
+// L_(x + 2 i, y + 2 (j - i), z) gives the others.
 // kmin: coefficients below it are not computed (zero): a Hessian-only product
 // has no degree-1 partials (kmin 3).
 template <int Q>
 __global__ void k_fmm_l2l(FmmLevel lv, FmmLevel lp, int has_parent, const int32_t* __restrict__ occ,
                           const float* __restrict__ Lpart, int chunks, float* __restrict__ L,
                           const double* __restrict__ done, int kmin) {
-  constexpr int NC = ncoef(Q) - 1;
+  constexpr int NC = ncoef(Q) - 1, NH = nharm(Q);
   if (done && *done != 0.0) return;
   const float* Lpar = L + lp.box_off * NC;
   float* Lout = L + lv.box_off * NC;
@@ -496,9 +565,16 @@ __global__ void k_fmm_l2l(FmmLevel lv, FmmLevel lp, int has_parent, const int32_
     const int64_t b = t % lv.nbox;
     float v = 0.f;
     if (k >= kmin && occ[lv.box_off + b] > 0) {
-      for (int ch = 0; ch < chunks; ++ch) v += Lpart[(int64_t(ch) * NC + k) * lv.nbox + b];
+      const char4 e = c_mi[k + 1];
+      const int j = e.z >> 1, z = e.z & 1;
+      for (int i = 0; i <= j; ++i) {
+        const float* lp = Lpart + int64_t(hidx(e.x + 2 * i, e.y + 2 * (j - i), z)) * lv.nbox + b;
+        float p = 0.f;
+        for (int ch = 0; ch < chunks; ++ch) p += lp[int64_t(ch) * NH * lv.nbox];
+        v += binom_f(j, i) * p;
+      }
+      if (j & 1) v = -v;
       if (has_parent) {
-        const char4 e = c_mi[k + 1];
         const int deg = e.x + e.y + e.z;
         const int x = int(b % lv.nx), y = int((b / lv.nx) % lv.ny), z = int(b / (int64_t(lv.nx) * lv.ny));
         const int64_t pb = (int64_t(z >> 1) * lp.ny + (y >> 1)) * lp.nx + (x >> 1);
@@ -1310,7 +1386,7 @@ mf_status Fmm::build(const float4* pos4, int64_t n, const float4* tpos4, int64_t
   // Interaction lists, rows and the derivative table are uploaded only when
   // they changed (positions that move a little keep the same grid shape).
   // Uploads go through pinned staging that stays alive until the next build.
-  const int NG = ncoef(Q + 1);
+  const int ND = ndtab(Q);
   std::vector<int32_t> dkey;
   dkey.reserve(did.size() * 3 + 1);
   dkey.push_back(Q);
@@ -1325,12 +1401,15 @@ mf_status Fmm::build(const float4* pos4, int64_t n, const float4* tpos4, int64_t
     // Kernels of earlier products may still read the old tables: the
     // uploads are ordered on the stream, from host copies kept as members.
     MF_CUDA_TRY(cudaStreamSynchronize(st));
-    host_dt_.assign(did.size() * size_t(NG), 0.f);
+    host_dt_.assign(did.size() * size_t(ND), 0.f);
     std::vector<double> D;
     for (const auto& kv : did) {
       const double R[3] = {double(std::get<0>(kv.first)), double(std::get<1>(kv.first)), double(std::get<2>(kv.first))};
       taylor_inv_r(R, Q + 1, D);
-      for (int g = 0; g < NG; ++g) host_dt_[size_t(kv.second) * NG + g] = float(D[size_t(g)]);
+      for (int n = 0; n <= Q + 1; ++n)
+        for (int z = 0; z <= std::min(n, 2); ++z)
+          for (int y = 0; y <= n - z; ++y)
+            host_dt_[size_t(kv.second) * size_t(ND) + size_t(didx(n - z - y, y, z))] = float(D[size_t(gidx(n - z - y, y, z))]);
     }
     MF_TRY(dtab_.reserve_slack(std::max<size_t>(1, host_dt_.size()) * sizeof(float)));
     if (!host_dt_.empty())
@@ -1373,9 +1452,10 @@ mf_status Fmm::build(const float4* pos4, int64_t n, const float4* tpos4, int64_t
     for (int cls = 0; cls < 8; ++cls) maxcnt = std::max(maxcnt, list_cnt_[size_t(8 * l + cls)]);
     ch = std::max<int64_t>(1, std::min<int64_t>({ch, 16, maxcnt}));
     chunks_[size_t(l)] = int32_t(ch);
-    lpart = std::max(lpart, ch * NC * v.nbox);
+    lpart = std::max(lpart, ch * nharm(Q) * v.nbox);
   }
   MF_TRY(mcoef_.reserve_slack(size_t(NC) * size_t(nbox_total) * sizeof(float)));
+  MF_TRY(hcoef_.reserve_slack(size_t(nharm(Q)) * size_t(nbox_total) * sizeof(float)));
   MF_TRY(lcoef_.reserve_slack(size_t(NC) * size_t(nbox_total) * sizeof(float)));
   MF_TRY(lpart_.reserve_slack(size_t(lpart) * sizeof(float)));
 
@@ -1440,82 +1520,6 @@ mf_status Fmm::product(int kind, const float4* pos4, const float4* smom, const A
 }
 
 namespace {
-// M2L launches of one level, split by local degree so the multipole and the
-// accumulators stay in registers.  hess: the product needs only the Hessian
-// of the local expansion (the Kelvin force, the force tensor), which no local
-// of degree 1 reaches (L2L maps degree >= 2 only from degree >= 2, and L2P of
-// the Hessian reads degree >= 2), so the degree-1 locals are not computed.
-template <int Q>
-struct M2LVariants;
-template <>
-struct M2LVariants<3> {
-  static void launch(const M2LArgs& p, unsigned g, cudaStream_t st, int* n, bool hess) {
-    if (hess) k_fmm_m2l<3, 2, 3><<<g, 128, 0, st>>>(p);
-    else k_fmm_m2l<3, 1, 3><<<g, 128, 0, st>>>(p);
-    *n += 1;
-  }
-};
-template <>
-struct M2LVariants<4> {
-  static void launch(const M2LArgs& p, unsigned g, cudaStream_t st, int* n, bool hess) {
-    if (hess) k_fmm_m2l<4, 2, 4><<<g, 128, 0, st>>>(p);
-    else k_fmm_m2l<4, 1, 4><<<g, 128, 0, st>>>(p);
-    *n += 1;
-  }
-};
-template <>
-struct M2LVariants<5> {
-  static void launch(const M2LArgs& p, unsigned g, cudaStream_t st, int* n, bool hess) {
-    if (hess) k_fmm_m2l<5, 2, 5><<<g, 128, 0, st>>>(p);
-    else k_fmm_m2l<5, 1, 5><<<g, 128, 0, st>>>(p);
-    *n += 1;
-  }
-};
-template <>
-struct M2LVariants<6> {
-  static void launch(const M2LArgs& p, unsigned g, cudaStream_t st, int* n, bool hess) {
-    if (hess) k_fmm_m2l<6, 2, 2><<<g, 128, 0, st>>>(p);
-    else k_fmm_m2l<6, 1, 2><<<g, 128, 0, st>>>(p);
-    k_fmm_m2l<6, 3, 6><<<g, 128, 0, st>>>(p);
-    *n += 2;
-  }
-};
-template <>
-struct M2LVariants<7> {
-  static void launch(const M2LArgs& p, unsigned g, cudaStream_t st, int* n, bool hess) {
-    if (hess) k_fmm_m2l<7, 2, 3><<<g, 128, 0, st>>>(p);
-    else k_fmm_m2l<7, 1, 3><<<g, 128, 0, st>>>(p);
-    k_fmm_m2l<7, 4, 7><<<g, 128, 0, st>>>(p);
-    *n += 2;
-  }
-};
-template <>
-struct M2LVariants<8> {
-  static void launch(const M2LArgs& p, unsigned g, cudaStream_t st, int* n, bool hess) {
-    if (hess) {
-      k_fmm_m2l<8, 2, 3><<<g, 128, 0, st>>>(p);
-      k_fmm_m2l<8, 4, 5><<<g, 128, 0, st>>>(p);
-      k_fmm_m2l<8, 6, 8><<<g, 128, 0, st>>>(p);
-    } else {
-      k_fmm_m2l<8, 1, 2><<<g, 128, 0, st>>>(p);
-      k_fmm_m2l<8, 3, 4><<<g, 128, 0, st>>>(p);
-      k_fmm_m2l<8, 5, 8><<<g, 128, 0, st>>>(p);
-    }
-    *n += 3;
-  }
-};
-template <>
-struct M2LVariants<9> {
-  // The force products only (Fmm::product refuses a field product at degree 9).
-  static void launch(const M2LArgs& p, unsigned g, cudaStream_t st, int* n, bool hess) {
-    if (!hess) return;
-    k_fmm_m2l<9, 2, 3><<<g, 128, 0, st>>>(p);
-    k_fmm_m2l<9, 4, 5><<<g, 128, 0, st>>>(p);
-    k_fmm_m2l<9, 6, 7><<<g, 128, 0, st>>>(p);
-    k_fmm_m2l<9, 8, 9><<<g, 128, 0, st>>>(p);
-    *n += 4;
-  }
-};
 // One CTA of 128 threads per leaf box, 256-source stages, also for small
 // boxes: 64 threads with 128-source stages measured slower at 262,144
 // particles (boxes of <= 40: near field 3.9 against 2.7 ms for the field,
@@ -1537,7 +1541,9 @@ mf_status Fmm::product_q(int kind, const float4* pos4, const float4* smom, const
   int32_t* occ = occ_.as<int32_t>();
   const int32_t* cnt = occ + leaf.box_off;
   const int32_t* tocc = separate_ ? tocc_.as<int32_t>() : occ;
+  constexpr int NH = nharm(Q);
   float* M = mcoef_.as<float>();
+  float* H = hcoef_.as<float>();  // multipoles with z <= 1
   float* Lc = lcoef_.as<float>();
   int nl = 0;
   if (marks) MF_CUDA_TRY(cudaEventRecord(marks[0], st));
@@ -1553,16 +1559,23 @@ mf_status Fmm::product_q(int kind, const float4* pos4, const float4* smom, const
         lv_[size_t(l + 1)], lv_[size_t(l)], occ, M, done);
     ++nl;
   }
+  {
+    FmmLevels lvs{};
+    for (int l = 0; l <= L; ++l) lvs.lv[l] = lv_[size_t(l)];
+    const dim3 grid{blocks_for(int64_t(NH) * leaf.nbox, 256, int64_t(sms) * 32), unsigned(L - 1)};
+    k_fmm_reduce<Q><<<grid, 256, 0, st>>>(lvs, 2, M, H, done);
+    ++nl;
+  }
   for (int l = 2; l <= L; ++l) {
     const FmmLevel& v = lv_[size_t(l)];
     M2LArgs p{};
     p.lv = v;
     p.occ = occ;
     p.tocc = tocc;
-    p.M = M + v.box_off * NC;
+    p.M = H + v.box_off * NH;
     p.Lp = lpart_.as<float>();
     p.list = lists_.as<int4>();
-    p.dtab = dtab_.as<float>();
+    p.dtab = dtab_.as<float4>();
     for (int cls = 0; cls < 8; ++cls) {
       p.list_off[cls] = list_off_[size_t(8 * l + cls)];
       p.list_cnt[cls] = int32_t(list_cnt_[size_t(8 * l + cls)]);
@@ -1574,7 +1587,13 @@ mf_status Fmm::product_q(int kind, const float4* pos4, const float4* smom, const
     p.per_class = ((int64_t(p.hx) * p.hy * p.hz) + 31) / 32 * 32;
     p.done = done;
     const int64_t threads = int64_t(p.chunks) * 8 * p.per_class;
-    M2LVariants<Q>::launch(p, unsigned((threads + 127) / 128), st, &nl, kind != 0);
+    // The products that need only the Hessian of the local expansion (the
+    // Kelvin force, the force tensor) leave out the degree-1 locals: no degree
+    // below 2 reaches it (L2L maps degree >= 2 only from degree >= 2).
+    const unsigned g = unsigned((threads + 127) / 128);
+    if (kind != 0) k_fmm_m2l<Q, 2><<<g, 128, 0, st>>>(p);
+    else if constexpr (Q <= kMaxFieldDegree) k_fmm_m2l<Q, 1><<<g, 128, 0, st>>>(p);
+    ++nl;
     k_fmm_l2l<Q><<<blocks_for(int64_t(NC) * v.nbox, 256, int64_t(sms) * 32), 256, 0, st>>>(
         v, lv_[size_t(l - 1)], l > 2 ? 1 : 0, tocc, lpart_.as<float>(), p.chunks, Lc, done, kind != 0 ? 3 : 0);
     ++nl;

@@ -518,7 +518,7 @@ class Fmm {
   int n_hrows_ = 0, n_off_ = 0;  // half-stencil rows and their box offsets (sym_near)
   int launches_ = 0;
   DevBuf cell_of_, cnt_, start_, cursor_, perm_tmp_, perm_, pos2s_, mom2s_;
-  DevBuf occ_, mcoef_, lcoef_, lpart_, lists_, rows_, dtab_, stat_, lofs_;
+  DevBuf occ_, mcoef_, hcoef_, lcoef_, lpart_, lists_, rows_, dtab_, stat_, lofs_;
   DevBuf hrows_, npart_;  // half-stencil rows; near-field partial sums (sym_near)
   // Separate targets: occupancy per level and leaf binning.
   DevBuf tocc_, tcell_of_, tstart_, tcursor_, tperm_tmp_, tperm_;
