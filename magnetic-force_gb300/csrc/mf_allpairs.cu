@@ -179,6 +179,38 @@ int device_sms(int device) {
 // ---------------------------------------------------------------------------
 // Kernel selection
 // ---------------------------------------------------------------------------
+template <class Real>
+AllPairsArgs<Real> allpairs_args(const Plan<Real>& plan, const LaunchIO<Real>& io, double* partials,
+                                 int32_t* counters, int32_t* err) {
+  AllPairsArgs<Real> a;
+  memset(&a, 0, sizeof(a));
+  a.scenes = plan.d_scenes.template as<SceneDesc<Real>>();
+  a.n_scenes = plan.n_scenes;
+  a.total_steps = plan.total_steps;
+  a.tpos = io.tpos;
+  a.tmom = io.tmom;
+  a.spos = io.spos;
+  a.smom = io.smom;
+  for (int k = 0; k < 9; ++k) {
+    a.out[k] = io.out[k];
+    a.rext[k] = io.rext[k];
+  }
+  a.out4 = io.out4;
+  a.add4 = io.add4;
+  a.add4b = io.add4b;
+  a.naive_quirks = io.naive_quirks;
+  a.done_flags = io.done_flags;
+  a.done_stride = io.done_stride;
+  a.corr4 = io.corr4;
+  a.done_count = io.done_count;
+  a.done_total = io.done_total;
+  a.partials = partials;
+  a.counters = counters;
+  a.err = err;
+  a.stage_wait_debug = stage_wait_debug();
+  return a;
+}
+
 template <class Real, Body B>
 struct BodyOf;
 template <class Real>
@@ -250,32 +282,7 @@ struct Launcher {
     if (plan.total_steps <= 0) return MF_OK;
     const int dev = current_device();
     const int64_t g = std::min<int64_t>(plan.total_steps, max_grid(dev));
-    AllPairsArgs<Real> a;
-    memset(&a, 0, sizeof(a));
-    a.scenes = plan.d_scenes.template as<SceneDesc<Real>>();
-    a.n_scenes = plan.n_scenes;
-    a.total_steps = plan.total_steps;
-    a.tpos = io.tpos;
-    a.tmom = io.tmom;
-    a.spos = io.spos;
-    a.smom = io.smom;
-    for (int k = 0; k < 9; ++k) {
-      a.out[k] = io.out[k];
-      a.rext[k] = io.rext[k];
-    }
-    a.out4 = io.out4;
-    a.add4 = io.add4;
-    a.add4b = io.add4b;
-    a.naive_quirks = io.naive_quirks;
-    a.done_flags = io.done_flags;
-    a.done_stride = io.done_stride;
-    a.corr4 = io.corr4;
-    a.done_count = io.done_count;
-    a.done_total = io.done_total;
-    a.partials = partials;
-    a.counters = counters;
-    a.err = err;
-    a.stage_wait_debug = stage_wait_debug();
+    const AllPairsArgs<Real> a = allpairs_args<Real>(plan, io, partials, counters, err);
     kernel()<<<unsigned(g), C::TPB, kSmem, st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "allpairs_kernel launch");
@@ -332,8 +339,10 @@ void fill_scene_coefs(const SceneSpec& s, SceneDesc<Real>& d) {
 
 template <class Real>
 mf_status build_plan(Body body, const std::vector<SceneSpec>& specs, Plan<Real>& plan, int shape) {
-  if constexpr (std::is_same<Real, float>::value)
-    if (shape == kShapeSym) return build_sym_plan(body, specs, plan);
+  if (shape == kShapeSym) {
+    if constexpr (std::is_same<Real, float>::value) return build_sym_plan(body, specs, plan);
+    else return build_sym64_plan(body, specs, plan);
+  }
   if (shape < 0 || shape >= kShapes || (shape != 0 && !(std::is_same<Real, float>::value && shaped(body))))
     return fail(MF_ERR_INVALID_ARG, "build_plan: bad block shape");
   int tile = 0, tbt = 0;
@@ -416,12 +425,12 @@ struct Shaped {
 
 template <class Real>
 void plan_scratch_needs(const Plan<Real>& plan, size_t* pd, size_t* nc) {
-  if constexpr (std::is_same<Real, float>::value)
-    if (plan.shape == kShapeSym) {
-      sym_needs(plan, pd);
-      *nc = 0;
-      return;
-    }
+  if (plan.shape == kShapeSym) {
+    if constexpr (std::is_same<Real, float>::value) sym_needs(plan, pd);
+    else *pd = sym64_partials(plan);
+    *nc = 0;
+    return;
+  }
   switch (plan.body) {
     case Body::Field: Shaped<Real, Body::Field>::needs(plan, pd, nc); break;
     case Body::Force: Shaped<Real, Body::Force>::needs(plan, pd, nc); break;
@@ -438,8 +447,10 @@ void plan_scratch_needs(const Plan<Real>& plan, size_t* pd, size_t* nc) {
 template <class Real>
 mf_status run_plan_raw(const Plan<Real>& plan, const LaunchIO<Real>& io, double* partials, int32_t* counters,
                        int32_t* err, cudaStream_t st) {
-  if constexpr (std::is_same<Real, float>::value)
-    if (plan.shape == kShapeSym) return run_sym(plan, io, partials, err, st);
+  if (plan.shape == kShapeSym) {
+    if constexpr (std::is_same<Real, float>::value) return run_sym(plan, io, partials, err, st);
+    else return run_sym64(plan, io, partials, err, st);
+  }
   switch (plan.body) {
     case Body::Field: return Shaped<Real, Body::Field>::launch(plan, io, partials, counters, err, st);
     case Body::Force: return Shaped<Real, Body::Force>::launch(plan, io, partials, counters, err, st);
@@ -619,6 +630,7 @@ std::string autotune_report() {
   template void fill_scene_coefs<R>(const SceneSpec&, SceneDesc<R>&);                                     \
   template mf_status refresh_plan_coefs<R>(const std::vector<SceneSpec>&, Plan<R>&);                      \
   template void plan_scratch_needs<R>(const Plan<R>&, size_t*, size_t*);                                  \
+  template AllPairsArgs<R> allpairs_args<R>(const Plan<R>&, const LaunchIO<R>&, double*, int32_t*, int32_t*); \
   template mf_status run_plan<R>(const Plan<R>&, const LaunchIO<R>&, Scratch&, cudaStream_t);             \
   template mf_status run_plan_raw<R>(const Plan<R>&, const LaunchIO<R>&, double*, int32_t*, int32_t*,     \
                                      cudaStream_t);

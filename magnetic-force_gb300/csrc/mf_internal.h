@@ -174,8 +174,9 @@ struct Shape {
 constexpr int kShapes = 5;
 constexpr Shape kShapeTable[kShapes] = {{256, 2, 256}, {128, 2, 256}, {256, 1, 256}, {128, 4, 128}, {128, 4, 256}};
 inline bool shaped(Body b) { return b != Body::Tensor; }
-// Shape index of the packed field / force evaluated once per unordered pair
-// (mf_sympair.cu), for scenes whose targets are their sources.
+// Shape index of the products evaluated once per unordered pair, for scenes
+// whose targets are their sources: the packed FP32 field / force
+// (mf_sympair.cu) and the FP64 ones (mf_sym64.cu).
 constexpr int kShapeSym = kShapes;
 
 // One scene of a launch before it is laid out in step space.  nt > 0, ns > 0.
@@ -193,7 +194,7 @@ struct SceneSpec {
 template <class Real>
 struct Plan {
   Body body = Body::Field;
-  int shape = 0;  // FP32 shaped bodies: index into kShapeTable, or kShapeSym
+  int shape = 0;  // FP32 shaped bodies: index into kShapeTable; kShapeSym (both precisions)
   int64_t total_steps = 0;
   int64_t total_tb = 0;
   int32_t n_scenes = 0;
@@ -257,6 +258,20 @@ mf_status build_sym_plan(Body body, const std::vector<SceneSpec>& specs, Plan<fl
 void sym_needs(const Plan<float>& plan, size_t* partial_doubles);
 mf_status run_sym(const Plan<float>& plan, const LaunchIO<float>& io, double* partials, int32_t* err,
                   cudaStream_t st);
+
+// The arguments of a launch of `plan` on io (all fields set).
+template <class Real>
+AllPairsArgs<Real> allpairs_args(const Plan<Real>& plan, const LaunchIO<Real>& io, double* partials,
+                                 int32_t* counters, int32_t* err);
+
+// The FP64 field and force once per unordered pair (mf_sym64.cu; FP64 plans
+// of shape kShapeSym): one scene whose targets are its sources.  The scratch
+// holds FP64 block sums (sym64_partials doubles).
+bool sym64_eligible(Body body, const std::vector<SceneSpec>& specs);
+mf_status build_sym64_plan(Body body, const std::vector<SceneSpec>& specs, Plan<double>& plan);
+size_t sym64_partials(const Plan<double>& plan);
+mf_status run_sym64(const Plan<double>& plan, const LaunchIO<double>& io, double* partials, int32_t* err,
+                    cudaStream_t st);
 
 // The field and the Kelvin force of the same dipoles once per unordered pair
 // in one launch (mf_sympair.cu).  The plan is a packed field plan (its

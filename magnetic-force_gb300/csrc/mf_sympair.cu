@@ -687,34 +687,6 @@ mf_status ff_grid(int* out) {
   return MF_OK;
 }
 
-AllPairsArgs<float> sym_args(const Plan<float>& plan, const LaunchIO<float>& io, int32_t* err) {
-  AllPairsArgs<float> a;
-  memset(&a, 0, sizeof(a));
-  a.scenes = plan.d_scenes.as<SceneDesc<float>>();
-  a.n_scenes = plan.n_scenes;
-  a.total_steps = plan.total_steps;
-  a.tpos = io.tpos;
-  a.tmom = io.tmom;
-  a.spos = io.spos;
-  a.smom = io.smom;
-  for (int k = 0; k < 9; ++k) {
-    a.out[k] = io.out[k];
-    a.rext[k] = io.rext[k];
-  }
-  a.out4 = io.out4;
-  a.add4 = io.add4;
-  a.add4b = io.add4b;
-  a.naive_quirks = io.naive_quirks;
-  a.done_flags = io.done_flags;
-  a.done_stride = io.done_stride;
-  a.corr4 = io.corr4;
-  a.done_count = io.done_count;
-  a.done_total = io.done_total;
-  a.err = err;
-  a.stage_wait_debug = stage_wait_debug();
-  return a;
-}
-
 }  // namespace
 
 bool sym_eligible(Body body, const std::vector<SceneSpec>& specs) {
@@ -787,7 +759,7 @@ mf_status run_sym(const Plan<float>& plan, const LaunchIO<float>& io, double* pa
   const bool force = plan.body == Body::ForceF2;
   int gmax = 0;
   MF_TRY(sym_grid(plan.body, &gmax));
-  const AllPairsArgs<float> a = sym_args(plan, io, err);
+  const AllPairsArgs<float> a = allpairs_args<float>(plan, io, nullptr, nullptr, err);
   float* part = reinterpret_cast<float*>(partials);
   const int64_t g = std::min<int64_t>(plan.total_steps, gmax);
   const int64_t g0 = plan.host.front().t_off;
@@ -824,7 +796,7 @@ mf_status run_symff(const Plan<float>& plan, const LaunchIO<float>& io, double* 
     return fail(MF_ERR_INVALID_ARG, "run_symff: not a field-and-force plan");
   int gmax = 0;
   MF_TRY(ff_grid(&gmax));
-  const AllPairsArgs<float> a = sym_args(plan, io, err);
+  const AllPairsArgs<float> a = allpairs_args<float>(plan, io, nullptr, nullptr, err);
   float* partf = reinterpret_cast<float*>(partials);
   float* partg = partf + size_t(plan.total_tb) * 3 * kFfTB;
   const int64_t g = std::min<int64_t>(plan.total_steps, gmax);
@@ -850,7 +822,7 @@ mf_status run_sym_force_from_sums(const Plan<float>& plan, const LaunchIO<float>
                                   const double* kept, const double* rows, int row_stride, int c_index, int32_t* err,
                                   cudaStream_t st) {
   if (plan.host.empty()) return MF_OK;
-  const AllPairsArgs<float> a = sym_args(plan, io, err);
+  const AllPairsArgs<float> a = allpairs_args<float>(plan, io, nullptr, nullptr, err);
   const int64_t g0 = plan.host.front().t_off;
   const int64_t n_span = plan.host.back().t_off + plan.host.back().nt - g0;
   const int64_t fb = std::min<int64_t>((n_span + 255) / 256, 8192);
