@@ -32,7 +32,7 @@ namespace mfgb {
 
 // The fitted force curves for the FP32 exact-branch body (staged into shared
 // memory by each CTA).
-static __constant__ float c_fit_ap[40] = MF_FITTED_CURVE_TABLE;
+static __constant__ ForceTable c_fit_ap = make_force_table();
 
 template <class Real>
 struct SceneDesc {
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(TPB) allpairs_kernel(const AllPairsArgs<Real> 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES];
   __shared__ int s_flag;
-  __shared__ float s_fit[40];
+  __shared__ __align__(16) float s_fit[80];
 
   const int tid = threadIdx.x;
   const int64_t T = a.total_steps;
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(TPB) allpairs_kernel(const AllPairsArgs<Real> 
     for (int s = 0; s < STAGES; ++s) mbar_init(&full_bar[s], 1);
     fence_mbar_init();
   }
-  if (tid < 40) s_fit[tid] = c_fit_ap[tid];
+  for (int k = tid; k < 80; k += TPB) s_fit[k] = c_fit_ap.v[k];
   __syncthreads();
 
   // Producer (thread 0): stage the source tile of step k into stage s.

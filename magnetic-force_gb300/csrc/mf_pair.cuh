@@ -35,7 +35,9 @@ constexpr double kInv4Pi = 1.0 / (4.0 * kPi);
 template <class Real>
 struct PairConsts {
   Real inv_h;        // 1/h
+  Real h;            // smoothing length
   Real ih3;          // 1/h^3
+  Real ih5;          // 1/h^5
   Real ih4_over_k;   // 1/(h^4 K): scales the fitted curves into the K-free form
   Real near2_field;  // (2h)^2: field pairs closer than this take the SPH branch
   Real near2_force;  // (4h)^2: force pairs at or inside this take the fitted branch
@@ -48,7 +50,9 @@ template <class Real>
 __host__ __device__ inline PairConsts<Real> make_pair_consts(double h) {
   PairConsts<Real> k;
   k.inv_h = Real(1.0 / h);
+  k.h = Real(h);
   k.ih3 = Real(1.0 / (h * h * h));
+  k.ih5 = Real(1.0 / (h * h * h * h * h));
   k.ih4_over_k = Real(1.0 / (h * h * h * h * kForceK));
   k.near2_field = Real(4.0 * h * h);
   k.near2_force = Real(16.0 * h * h);
@@ -295,56 +299,103 @@ __device__ __forceinline__ void clamped_force_coeffs(float near2, float& P, floa
   Q = ri2 * -5.f * P;
 }
 
-// Branch-free FP32 forms of the near-field coefficients for the correction
-// pass, where lanes of a warp sit on different branches: both SPH pieces are
-// evaluated and selected; the fitted-curve piece is looked up in a 4 x 10
-// coefficient table (c1 then c2 of each piece, highest power first).
-// Same mathematics as field_near_coeffs / force_near_coeffs.
-__device__ __forceinline__ void field_near_coeffs_fast(float r2, float inv_h, float ih3, float& alpha, float& beta) {
-  const float ri = rsqrt_approx(r2);
-  const bool pos = r2 > 0.f;
-  const float r = pos ? r2 * ri : 0.f;
-  const float q = r * inv_h, q2 = q * q, q3 = q2 * q;
-  const float tmq = 2.f - q, tmq3 = tmq * tmq * tmq;
-  const float omq = 1.f - q;
-  const float Pq = q3 * (q3 * (1.f / 6.f) - q2 * (6.f / 5.f) + 3.f * q - 8.f / 3.f) + 1.f / 15.f;
-  float rq3;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rq3) : "f"(fmaxf(q3, 1.f)));
+// Branch-free FP32 forms of the near-field coefficients, for kernels where the
+// lanes of a warp sit on different pieces.  Same mathematics as
+// field_near_coeffs / force_near_coeffs with the polynomials multiplied out.
+
+// Field: alpha h^5 and beta h^3 at q = r / h < 2.  The outer piece's beta is
+// written in t = 2 - q, where its terms do not cancel (they vanish at q = 2):
+//   q < 1: 0.8 - 0.5 q,                        -8/3 + 4.8 q^2 - 2.5 q^3
+//   else:  q/6 - 0.8 + 1/q - q^-5/15,          2/15 + t/5 + t^2/5 - 5 t^3/6 - q^-3/15
+// ri: near_rsqrt(r2), finite at r = 0 (where q comes out 0).
+__device__ __forceinline__ float near_rsqrt(float r2) { return rsqrt_approx(fmaxf(r2, 1e-36f)); }
+__device__ __forceinline__ void field_near_unit(float r2, float ri, float h, float inv_h, float& al, float& be) {
+  const float q = (r2 * ri) * inv_h, iq = ri * h;
+  const float iq2 = iq * iq, iq3 = iq2 * iq, t = 2.f - q;
   const bool hi = q >= 1.f;
-  const float wa = hi ? -3.f * Pq * rq3 : (15.f * q3 - 36.f * q2 + 40.f) * 0.1f;
-  const float wd = hi ? tmq3 : tmq3 - 4.f * omq * omq * omq;
-  beta = (wa * (1.f / 3.f) - wd) * ih3;
-  alpha = pos ? (wa - wd) * ih3 * (1.f / 3.f) * (ri * ri) : 0.f;
+  const float al_hi = fmaf(q, 1.f / 6.f, iq - 0.8f) - (iq3 * iq2) * (1.f / 15.f);
+  const float be_hi = fmaf(t, fmaf(t, fmaf(t, -5.f / 6.f, 0.2f), 0.2f), 2.f / 15.f) - iq3 * (1.f / 15.f);
+  const float al_lo = fmaf(q, -0.5f, 0.8f);
+  const float be_lo = fmaf(q * q, fmaf(q, -2.5f, 4.8f), -8.f / 3.f);
+  al = hi ? al_hi : al_lo;
+  be = hi ? be_hi : be_lo;
 }
 
-__device__ __forceinline__ void force_near_coeffs_fast(float r2, const float* __restrict__ tbl, float inv_h,
-                                                       float ih4_over_k, float& P, float& Q) {
+// The same for two distances at once (packed FP32).
+__device__ __forceinline__ void field_near_unit2(float2 r2, float h, float inv_h, float2& al, float2& be) {
+  const float2 ri = make_float2(near_rsqrt(r2.x), near_rsqrt(r2.y));
+  const float2 q = f2_mul(f2_mul(r2, ri), f2_dup(inv_h)), iq = f2_mul(ri, f2_dup(h));
+  const float2 iq2 = f2_mul(iq, iq), iq3 = f2_mul(iq2, iq), t = f2_sub(f2_dup(2.f), q);
+  const float2 m15 = f2_dup(-1.f / 15.f);
+  const float2 al_hi = f2_fma(f2_mul(iq3, iq2), m15, f2_fma(q, f2_dup(1.f / 6.f), f2_add(iq, f2_dup(-0.8f))));
+  const float2 b3 = f2_fma(t, f2_fma(t, f2_dup(-5.f / 6.f), f2_dup(0.2f)), f2_dup(0.2f));
+  const float2 be_hi = f2_fma(iq3, m15, f2_fma(t, b3, f2_dup(2.f / 15.f)));
+  const float2 al_lo = f2_fma(q, f2_dup(-0.5f), f2_dup(0.8f));
+  const float2 be_lo = f2_fma(f2_mul(q, q), f2_fma(q, f2_dup(-2.5f), f2_dup(4.8f)), f2_dup(-8.f / 3.f));
+  const bool h0 = q.x >= 1.f, h1 = q.y >= 1.f;
+  al = make_float2(h0 ? al_hi.x : al_lo.x, h1 ? al_hi.y : al_lo.y);
+  be = make_float2(h0 ? be_hi.x : be_lo.x, h1 ? be_hi.y : be_lo.y);
+}
+
+// The fitted-curve table for the force (Dipole_hessian.kern:53-61) in the
+// layout force_curves reads from shared memory: entry i = ceil(q) of three
+// arrays, (C1's q^4 .. q^1), (C2's q^4 .. q^1), (both constants).  Entries 0
+// and 1 hold the piece q <= 1, 2 and 3 the next two, the others q > 3 (any
+// index of three bits is inside the table).
+struct ForceTable {
+  float v[80];
+};
+constexpr ForceTable make_force_table() {
+  constexpr double c[4][10] = {
+      {9.97813616438174e-09, -2.97897856524718e-08, 2.38918644566813e-09, 4.53199938857366e-08,
+       2.44617454752747e-11, 6.69550479838731e-08, -1.61753307173877e-07, 1.68213714992711e-08,
+       1.34558143036838e-07, 1.10976027980100e-10},
+      {-2.76473728643294e-09, 2.86975546540539e-08, -9.94582836806651e-08, 1.25129924573675e-07,
+       -2.37010166723652e-08, -3.08460139955194e-08, 2.29192245602275e-07, -5.88399621128587e-07,
+       5.61170054591844e-07, -1.14421132829680e-07},
+      {-1.09679990621465e-09, 9.77055663264614e-09, -2.54781238661150e-08, 2.65020634884934e-09,
+       5.00787562417835e-08, 3.50477408060213e-09, -5.25956271895141e-08, 2.78876509535747e-07,
+       -6.24199554212217e-07, 4.91807818904985e-07},
+      {3.79927162333632e-10, -6.26368404962679e-09, 3.94760528277489e-08, -1.13580541622200e-07,
+       1.27491333574323e-07, 7.33485346367840e-10, -9.58855788627803e-09, 4.37085309763591e-08,
+       -7.48004594092261e-08, 2.34161209605651e-08}};
+  ForceTable t{};
+  for (int i = 0; i < 8; ++i) {
+    const int p = i < 1 ? 0 : i > 4 ? 3 : i - 1;
+    for (int k = 0; k < 4; ++k) {
+      t.v[4 * i + k] = float(c[p][k]);
+      t.v[32 + 4 * i + k] = float(c[p][5 + k]);
+    }
+    t.v[64 + 2 * i] = float(c[p][4]);
+    t.v[64 + 2 * i + 1] = float(c[p][9]);
+  }
+  return t;
+}
+
+// C1(q) and C2(q) for 0 <= q <= 4 (C2 - 3 C1 is formed from the two values: as
+// curves of its own its rounding no longer cancelled C1's along d, and the
+// force came out 2.7e-6 instead of 1.1e-6 from the oracle).  tbl: a ForceTable in shared memory, 16-byte
+// aligned.  ceil(q) by one add rounded up to a whole number (no conversion
+// through the slow units).  Other q give values the caller must not use.
+__device__ __forceinline__ void force_curves(float q, const float* __restrict__ tbl, float& c1, float& c2) {
+  const int i = __float_as_int(__fadd_ru(q, 8388608.f)) & 7;
+  const float4 a = *reinterpret_cast<const float4*>(tbl + 4 * i);
+  const float4 b = *reinterpret_cast<const float4*>(tbl + 32 + 4 * i);
+  const float2 c = *reinterpret_cast<const float2*>(tbl + 64 + 2 * i);
+  c1 = fmaf(q, fmaf(q, fmaf(q, fmaf(q, a.x, a.y), a.z), a.w), c.x);
+  c2 = fmaf(q, fmaf(q, fmaf(q, fmaf(q, b.x, b.y), b.z), b.w), c.y);
+}
+
+// (P, Q) of the force tensor for 0 < r <= 4h, in units of K.
+__device__ __forceinline__ void force_near_pq(float r2, const float* __restrict__ tbl, float inv_h, float ih4_over_k,
+                                              float& P, float& Q) {
   const float ri = rsqrt_approx(r2);
-  const bool pos = r2 > 0.f;
-  const float r = pos ? r2 * ri : 0.f;
-  const float q = fminf(r * inv_h, 4.f);
-  const int piece = min(max(int(ceilf(q)) - 1, 0), 3);
-  const float* c = tbl + piece * 10;
-  const float c1 = q * (q * (q * (q * c[0] + c[1]) + c[2]) + c[3]) + c[4];
-  const float c2 = q * (q * (q * (q * c[5] + c[6]) + c[7]) + c[8]) + c[9];
+  float c1, c2;
+  force_curves((r2 * ri) * inv_h, tbl, c1, c2);
   const float s = ih4_over_k * ri;
-  P = pos ? c1 * s : 0.f;
-  Q = pos ? (c2 - 3.f * c1) * s * (ri * ri) : 0.f;
+  P = c1 * s;
+  Q = fmaf(-3.f, c1, c2) * s * (ri * ri);
 }
-
-// The fitted-curve table in the layout force_near_coeffs_fast reads
-// (Dipole_hessian.kern:53-61): per piece, C1 then C2, highest power first.
-#define MF_FITTED_CURVE_TABLE                                                                      \
-  {9.97813616438174e-09f,  -2.97897856524718e-08f, 2.38918644566813e-09f,  4.53199938857366e-08f,  \
-   2.44617454752747e-11f,  6.69550479838731e-08f,  -1.61753307173877e-07f, 1.68213714992711e-08f,  \
-   1.34558143036838e-07f,  1.10976027980100e-10f,  -2.76473728643294e-09f, 2.86975546540539e-08f,  \
-   -9.94582836806651e-08f, 1.25129924573675e-07f,  -2.37010166723652e-08f, -3.08460139955194e-08f, \
-   2.29192245602275e-07f,  -5.88399621128587e-07f, 5.61170054591844e-07f,  -1.14421132829680e-07f, \
-   -1.09679990621465e-09f, 9.77055663264614e-09f,  -2.54781238661150e-08f, 2.65020634884934e-09f,  \
-   5.00787562417835e-08f,  3.50477408060213e-09f,  -5.25956271895141e-08f, 2.78876509535747e-07f,  \
-   -6.24199554212217e-07f, 4.91807818904985e-07f,  3.79927162333632e-10f,  -6.26368404962679e-09f, \
-   3.94760528277489e-08f,  -1.13580541622200e-07f, 1.27491333574323e-07f,  7.33485346367840e-10f,  \
-   -9.58855788627803e-09f, 4.37085309763591e-08f,  -7.48004594092261e-08f, 2.34161209605651e-08f}
 
 // FP32 exact pair forms without a branch: the far coefficients and the fast
 // near coefficients above are both evaluated and selected by the radius, so
@@ -354,12 +405,12 @@ __device__ __forceinline__ void force_near_coeffs_fast(float r2, const float* __
 __device__ __forceinline__ void field_pair_sel(float dx, float dy, float dz, float sx, float sy, float sz,
                                                const PairConsts<float>& k, float* s1, float* s2) {
   const float r2 = dx * dx + dy * dy + dz * dz;
+  const float ri = near_rsqrt(r2), ri2 = ri * ri, ri3 = ri2 * ri;
   float al, be;
-  field_near_coeffs_fast(r2, k.inv_h, k.ih3, al, be);
-  const float ri = rsqrt_approx(r2), ri2 = ri * ri, ri3 = ri2 * ri;
+  field_near_unit(r2, ri, k.h, k.inv_h, al, be);
   const bool far = r2 >= k.near2_field;
-  const float beta = far ? ri3 : be;
-  const float alpha = far ? ri3 * ri2 : al;
+  const float beta = far ? ri3 : be * k.ih3;
+  const float alpha = far ? ri3 * ri2 : al * k.ih5;
   const float t = (dx * sx + dy * sy + dz * sz) * alpha;
   s1[0] += dx * t;
   s1[1] += dy * t;
@@ -376,11 +427,11 @@ __device__ __forceinline__ void force_pair_sel(float dx, float dy, float dz, flo
   const float dm = dx * mx + dy * my + dz * mz;
   const float sm = sx * mx + sy * my + sz * mz;
   float Pn, Qn;
-  force_near_coeffs_fast(r2, k.tbl, k.inv_h, k.ih4_over_k, Pn, Qn);
+  force_near_pq(r2, k.tbl, k.inv_h, k.ih4_over_k, Pn, Qn);
   const float ri = rsqrt_approx(r2), ri2 = ri * ri, ri5 = ri2 * ri2 * ri;
-  const bool far = r2 > k.near2_force;
-  const float P = far ? ri5 : Pn;
-  const float Q = far ? -5.f * ri5 * ri2 : Qn;
+  const bool far = r2 > k.near2_force, apart = r2 > 0.f;
+  const float P = far ? ri5 : apart ? Pn : 0.f;
+  const float Q = far ? -5.f * ri5 * ri2 : apart ? Qn : 0.f;
   const float u = P * ds, v = P * dm, w = P * sm + Q * ds * dm;
   f[0] += dx * w + mx * u + sx * v;
   f[1] += dy * w + my * u + sy * v;
