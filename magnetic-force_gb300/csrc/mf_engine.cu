@@ -1165,8 +1165,7 @@ class Engine final : public EngineBase {
 
   template <class Op>
   mf_status reduce(const Op& op) {
-    const int64_t gx = grid_1d(np_, sms_) > unsigned(sms_ * 2) ? sms_ * 2 : grid_1d(np_, sms_);
-    dim3 grid(unsigned(gx), 1);
+    const dim3 grid(grid_1d(np_, sms_), 1);
     reduce_kernel<Op><<<grid, 256, 0, st_>>>(op, range_.template as<VecRange>(), scal_.template as<double>(),
                                              red_part_.template as<double>(), red_ticket_.template as<int32_t>());
     MF_CUDA_TRY(cudaGetLastError());

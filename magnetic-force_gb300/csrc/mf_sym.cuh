@@ -90,18 +90,18 @@ __device__ __forceinline__ void sym_field_pair2(float2 tx, float2 ty, float2 tz,
 // are formed once (54 packed operations per target and item against 30 + 36
 // apart).  Each term is the one sym_field_pair2 / sym_force_pair2 forms,
 // operation for operation: the field clamped at its near radius (nf2), the
-// force at its own (ng2).
+// force at its own, beyond which 1/r is at most rg = rsqrt_approx(4h squared).
 __device__ __forceinline__ void sym_field_force_pair2(float2 tx, float2 ty, float2 tz, float2 tmx, float2 tmy,
-                                                      float2 tmz, const PairItems::Item& it, float nf2, float ng2,
+                                                      float2 tmz, const PairItems::Item& it, float nf2, float rg,
                                                       float2* accf, float2* accg, float2* srcf, float2* srcg) {
   const float2 dx = f2_sub(tx, it.x), dy = f2_sub(ty, it.y), dz = f2_sub(tz, it.z);
   const float2 r2 = f2_fma(dz, dz, f2_fma(dy, dy, f2_mul(dx, dx)));
   const float2 ds = f2_fma(dz, it.mz, f2_fma(dy, it.my, f2_mul(dx, it.mx)));
   const float2 dm = f2_fma(dz, tmz, f2_fma(dy, tmy, f2_mul(dx, tmx)));
+  const float2 rf = clamp_rsqrt2(r2, nf2);
   {
-    const float2 ri = clamp_rsqrt2(r2, nf2);
-    const float2 ri2 = f2_mul(ri, ri);
-    const float2 beta = f2_mul(ri2, ri);
+    const float2 ri2 = f2_mul(rf, rf);
+    const float2 beta = f2_mul(ri2, rf);
     const float2 a3 = f2_mul(beta, f2_mul(ri2, f2_dup(-3.f)));
     const float2 ts = f2_mul(ds, a3);
     const float2 tt = f2_mul(dm, a3);
@@ -113,7 +113,7 @@ __device__ __forceinline__ void sym_field_force_pair2(float2 tx, float2 ty, floa
     srcf[2] = f2_fma(tmz, beta, f2_fma(dz, tt, srcf[2]));
   }
   {
-    const float2 ri = clamp_rsqrt2(r2, ng2);
+    const float2 ri = make_float2(fminf(rf.x, rg), fminf(rf.y, rg));
     const float2 ri2 = f2_mul(ri, ri);
     const float2 ri5 = f2_mul(f2_mul(ri2, ri2), ri);
     const float2 sm = f2_fma(it.mz, tmz, f2_fma(it.my, tmy, f2_mul(it.mx, tmx)));

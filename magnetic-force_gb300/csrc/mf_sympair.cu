@@ -379,7 +379,10 @@ __global__ void k_sym_finish(const AllPairsArgs<float> a, const float* __restric
 // Measured at N = 65,536 / 131,072 (ms per fused launch with its finish;
 // targets per thread, CTAs per SM, phases): 4, 3, 2 (166 registers) 4.90 /
 // 18.54; 6, 2, 2 (242) 4.63 / 17.93; 8, 2, 4 (255, 124 bytes of spills)
-// 4.54 / 18.05.  The separate products take 5.36 / 21.37.
+// 4.54 / 18.05; with the force's clamp as a minimum of the field's 1/r (two
+// reciprocal square roots fewer per target and item) 4.43.  Unrolled 1 or 4
+// items deep instead of 2: 4.47 / 4.75.  The separate products take 5.36 /
+// 21.37.
 constexpr int kFfTPB = 128, kFfTPT = 8, kFfStages = 2, kFfMinBlocks = 2;
 constexpr int kFfTB = kFfTPB * kFfTPT;
 constexpr int kFfWarps = kFfTPB / 32;
@@ -468,7 +471,7 @@ __global__ void __launch_bounds__(kFfTPB, kFfMinBlocks) k_sym_ff(const AllPairsA
       const int n_items = PairItems::items(cnt);
       const float4* __restrict__ sp = stage_pos(s);
       const float4* __restrict__ smv = stage_mom(s);
-      const float nf2 = sc.pc.near2_field, ng2 = sc.pc.near2_force;
+      const float nf2 = sc.pc.near2_field, rg = rsqrt_approx(sc.pc.near2_force);
       const float kf = -float(kInv4Pi), kg = float(kForceK);
       float2 accf[TPT][3], accg[TPT][3];
 #pragma unroll
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(kFfTPB, kFfMinBlocks) k_sym_ff(const AllPairsA
           float2 srcg[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
           for (int t = 0; t < TPT; ++t)
-            sym_field_force_pair2(tx[t], ty[t], tz[t], tmx[t], tmy[t], tmz[t], it, nf2, ng2, accf[t], accg[t], srcf,
+            sym_field_force_pair2(tx[t], ty[t], tz[t], tmx[t], tmy[t], tmz[t], it, nf2, rg, accf[t], accg[t], srcf,
                                   srcg);
           if (sym) {  // warp-uniform
             float v[16];
