@@ -15,8 +15,8 @@
 //   * I < J: each thread holds TPT targets of block I in registers and sweeps
 //     tile J (bulk-copied to shared memory on an mbarrier pipeline, 2 sources
 //     per packed f32x2 instruction).  Each pair adds into the target's sum
-//     and into the tile's source sums; those are reduced over the warp by a
-//     fixed shuffle tree and over the warps in a fixed order.
+//     and into the tile's source sums; those are summed over the warp by a
+//     rotation of the items over the lanes and over the warps in a fixed order.
 //   * I == J: the block against itself, every ordered pair, target side only.
 // Every step writes its FP32 block sums (scaled to the all-pairs kernels'
 // output units) into part[K][X] -- the sums for block K from partner block
@@ -39,16 +39,24 @@ constexpr int kSymTPB = 128, kSymTPT = 8, kSymStages = 2;
 constexpr int kSymTB = kSymTPB * kSymTPT;  // particles per block = sources per tile
 constexpr int kSymWarps = kSymTPB / 32;
 constexpr size_t kSymSmem = size_t(kSymStages) * 2 * kSymTB * sizeof(float4);
-// A tile's source sums are reduced over the warps in kSymSplit phases (the
-// per-warp buffer holds one phase: less shared memory per CTA), and over the
-// lanes kSymPair items at a time (one shuffle tree for 6 * kSymPair values).
-// Measured at N = 65,536 / 131,072 (ms per product; TPB x TPT, stages,
-// split, pair): 128x4 3,1,1 3.41 / 13.02; 128x4 2,2,2 3.23 / 12.66;
-// 128x4 2,2,4 3.14 / 12.31; 128x8 2,2,1 3.01 / 12.00; 128x8 2,4,2 2.94 /
-// 11.68; 64x8 2,2,2 2.95 / 11.56; 128x8 2,2,2 2.88 / 11.47 (254 registers,
-// 2 CTAs per SM).
-// (The field body sets its own split and pair counts below.)
-constexpr int kSymSplit = 2, kSymPair = 2;
+// A tile's source sums are added over the warps in kSymSplit phases (the
+// per-warp buffer holds one phase: less shared memory per CTA).  Within a warp
+// they travel: at rotation r lane l meets item (l + r) & 31 of a group of 32,
+// adds its eight targets' terms into that item's sums and hands them to lane
+// l - 1, so after 32 rotations every lane holds one item's sums over the whole
+// warp.  A shuffle tree per pair of items took five times the instructions
+// (selects and adds of all its levels: 62 against 18 per item for both
+// products) and their register ports are what bounds these kernels: a packed
+// FMA with three different 64-bit operands takes 3 cycles of its 2-cycle slot.
+// Measured at N = 65,536 (ms per product with its finish; rotation against
+// tree): field 2.45 / 2.50, force 2.75 / 2.80, both in one launch 4.22 / 4.43.
+// Targets per thread with the rotation, CTAs per SM: 4, 4 (128 registers)
+// 2.56 / 2.92 (field / force); 6, 3 2.65 / 3.04; 8, 2 2.45 / 2.75: more warps
+// do not help.
+constexpr int kSymSplit = 2;
+// Floats per item in the buffer: 6 sums and one more, so that the lanes'
+// stores and the reads of 32 consecutive sources fall in distinct banks.
+constexpr int kSymRow = 7;
 
 // Step l of a scene with nb blocks -> (I, J), row I holding nb - I steps.
 __device__ __forceinline__ void sym_block_pair(int64_t l, int nb, int& I, int& J) {
@@ -75,7 +83,6 @@ struct SymBody<true> {
   // Targets from the AoS records (a force product always has them; reading
   // them from the pair records cost 3 % in the force kernel at N = 65,536).
   static constexpr bool kAosTargets = true;
-  static constexpr int kSplit = kSymSplit, kPair = kSymPair;
   __device__ static float near2(const PairConsts<float>& pc) { return pc.near2_force; }
   __device__ static float scale() { return float(kForceK); }
   __device__ static void pair(float2 tx, float2 ty, float2 tz, float2 tmx, float2 tmy, float2 tmz,
@@ -92,7 +99,6 @@ template <>
 struct SymBody<false> {
   static constexpr float kSrcSign = 1.f;
   static constexpr bool kAosTargets = false;  // a field product carries the pair records only
-  static constexpr int kSplit = 2, kPair = 2;
   __device__ static float near2(const PairConsts<float>& pc) { return pc.near2_field; }
   __device__ static float scale() { return -float(kInv4Pi); }
   __device__ static void pair(float2 tx, float2 ty, float2 tz, float2 tmx, float2 tmy, float2 tmz,
@@ -114,18 +120,15 @@ __device__ __forceinline__ bool scene_done(const AllPairsArgs<float>& a, const S
 }
 
 template <bool kForce>
-__global__ void __launch_bounds__(kSymTPB) k_sym(const AllPairsArgs<float> a, float* __restrict__ part) {
+__global__ void __launch_bounds__(kSymTPB, 2) k_sym(const AllPairsArgs<float> a, float* __restrict__ part) {
   using BodyT = SymBody<kForce>;
   constexpr int TPB = kSymTPB, TPT = kSymTPT, TB = kSymTB, STAGES = kSymStages;
-  constexpr int SPLIT = BodyT::kSplit, NH = TB / 2 / SPLIT, P = BodyT::kPair;
-  constexpr int NV = P * 6 <= 8 ? 8 : (P * 6 <= 16 ? 16 : 32);
-  static_assert(NH % P == 0, "phase items");
+  constexpr int SPLIT = kSymSplit, NH = TB / 2 / SPLIT;
+  static_assert(NH % 32 == 0, "phases of whole groups of 32 items");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES];
   // per warp: the source sums of the phase's pair items, [item][component * 2 + source of the pair]
-  // (row stride 6: the lanes' writes of one item, and 32 threads' reads of
-  // consecutive sources, fall in distinct banks)
-  __shared__ float s_srcf[kSymWarps][NH * 6];
+  __shared__ float s_srcf[kSymWarps][NH * kSymRow];
 
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int64_t T = a.total_steps, G = gridDim.x, b = blockIdx.x;
@@ -211,6 +214,11 @@ __global__ void __launch_bounds__(kSymTPB) k_sym(const AllPairsArgs<float> a, fl
       const int n_items = PairItems::items(cnt);
       const float4* __restrict__ sp = stage_pos(s);
       const float4* __restrict__ smv = stage_mom(s);
+      if (n_items & 31) {  // items past the tile's end, up to a whole group: zero dipoles
+        for (int k = 2 * n_items + tid; k < 2 * ((n_items + 31) & ~31); k += TPB)
+          stage_pos(s)[k] = stage_mom(s)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+      }
       const float near2 = BodyT::near2(sc.pc);
       const float kk = BodyT::scale();
       float2 acc[TPT][3];
@@ -218,33 +226,36 @@ __global__ void __launch_bounds__(kSymTPB) k_sym(const AllPairsArgs<float> a, fl
       for (int t = 0; t < TPT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = make_float2(0.f, 0.f);
       for (int h = 0; h < SPLIT; ++h) {
         const int j_end = min(n_items, (h + 1) * NH);
+        for (int j0 = h * NH; j0 < j_end; j0 += 32) {
+          // The source sums of item j0 + ((lane + r) & 31) at rotation r: every
+          // lane meets the group's 32 items in turn and hands their sums on.
+          float2 run[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) run[c] = make_float2(0.f, 0.f);
 #pragma unroll 2
-        for (int j0 = h * NH; j0 < j_end; j0 += P) {
-          float v[NV];
+          for (int r = 0; r < 32; ++r) {
+            const PairItems::Item it = PairItems::load_item(sp, smv, j0 + ((lane + r) & 31));
+            float2 src[3];
 #pragma unroll
-          for (int q = 0; q < NV; ++q) v[q] = 0.f;
-#pragma unroll
-          for (int p = 0; p < P; ++p) {
-            // An item past the tile's end is a zero dipole at the origin:
-            // nothing on the target side; its source-side sums belong to
-            // slots past the scene's end, which are never read.
-            const bool in = p == 0 || j0 + p < j_end;
-            const PairItems::Item it =
-                in ? PairItems::load_item(sp, smv, j0 + p) : PairItems::Item{{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f},
-                                                                            {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-            float2 src[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            for (int c = 0; c < 3; ++c) src[c] = make_float2(0.f, 0.f);
 #pragma unroll
             for (int t = 0; t < TPT; ++t) BodyT::pair(tx[t], ty[t], tz[t], tmx[t], tmy[t], tmz[t], it, near2, acc[t], src);
+            if (sym) {  // warp-uniform
+              const int from = (lane + 1) & 31;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              v[p * 6 + 2 * c] = src[c].x;
-              v[p * 6 + 2 * c + 1] = src[c].y;
+              for (int c = 0; c < 3; ++c) {
+                const float2 v = f2_add(run[c], src[c]);
+                run[c] = make_float2(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from));
+              }
             }
           }
-          if (sym) {  // warp-uniform
-            const float w = warp_reduce_scatter<NV>(v, lane);
-            const int kv = lane / (32 / NV);
-            if (lane % (32 / NV) == 0 && kv < 6 * P) s_srcf[wid][(j0 - h * NH) * 6 + kv] = w;
+          if (sym) {  // back at item `lane`
+            float* d = s_srcf[wid] + (j0 - h * NH + lane) * kSymRow;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              d[2 * c] = run[c].x;
+              d[2 * c + 1] = run[c].y;
+            }
           }
         }
         if (sym) {
@@ -258,7 +269,7 @@ __global__ void __launch_bounds__(kSymTPB) k_sym(const AllPairsArgs<float> a, fl
             for (int c = 0; c < 3; ++c) {
               float x = 0.f;
 #pragma unroll
-              for (int w = 0; w < kSymWarps; ++w) x += s_srcf[w][j * 6 + 2 * c + (r & 1)];
+              for (int w = 0; w < kSymWarps; ++w) x += s_srcf[w][j * kSymRow + 2 * c + (r & 1)];
               ps[c * TB + rr] = x * ks;
             }
           }
@@ -381,8 +392,9 @@ __global__ void k_sym_finish(const AllPairsArgs<float> a, const float* __restric
 // 18.54; 6, 2, 2 (242) 4.63 / 17.93; 8, 2, 4 (255, 124 bytes of spills)
 // 4.54 / 18.05; with the force's clamp as a minimum of the field's 1/r (two
 // reciprocal square roots fewer per target and item) 4.43.  Unrolled 1 or 4
-// items deep instead of 2: 4.47 / 4.75.  The separate products take 5.36 /
-// 21.37.
+// items deep instead of 2: 4.47 / 4.75.  With the source sums travelling from
+// lane to lane (kSymSplit above) 4.22; 4 targets, 3 CTAs 4.58, 6, 2 4.35.  The
+// separate products take 5.20.
 constexpr int kFfTPB = 128, kFfTPT = 8, kFfStages = 2, kFfMinBlocks = 2;
 constexpr int kFfTB = kFfTPB * kFfTPT;
 constexpr int kFfWarps = kFfTPB / 32;
@@ -390,7 +402,7 @@ constexpr size_t kFfSmem = size_t(kFfStages) * 2 * kFfTB * sizeof(float4);
 constexpr int kFfSplit = 4;  // phases per tile: the per-warp source sums of one phase fit the static smem
 constexpr int kFfNH = kFfTB / 2 / kFfSplit;  // pair items per phase
 // Per item, 12 source sums: field x, y, z then force x, y, z, each for the
-// item's two sources.  Row stride 13 (odd): one item's 12 lane writes, and
+// item's two sources.  Row stride 13 (odd): the lanes' writes of one sum, and
 // the phase-end reads of 32 consecutive sources, fall in distinct banks.
 constexpr int kFfRow = 13;
 
@@ -471,6 +483,11 @@ __global__ void __launch_bounds__(kFfTPB, kFfMinBlocks) k_sym_ff(const AllPairsA
       const int n_items = PairItems::items(cnt);
       const float4* __restrict__ sp = stage_pos(s);
       const float4* __restrict__ smv = stage_mom(s);
+      if (n_items & 31) {  // items past the tile's end, up to a whole group: zero dipoles
+        for (int k = 2 * n_items + tid; k < 2 * ((n_items + 31) & ~31); k += TPB)
+          stage_pos(s)[k] = stage_mom(s)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+      }
       const float nf2 = sc.pc.near2_field, rg = rsqrt_approx(sc.pc.near2_force);
       const float kf = -float(kInv4Pi), kg = float(kForceK);
       float2 accf[TPT][3], accg[TPT][3];
@@ -480,28 +497,38 @@ __global__ void __launch_bounds__(kFfTPB, kFfMinBlocks) k_sym_ff(const AllPairsA
         for (int c = 0; c < 3; ++c) accf[t][c] = accg[t][c] = make_float2(0.f, 0.f);
       for (int h = 0; h < SPLIT; ++h) {
         const int j_end = min(n_items, (h + 1) * NH);
+        for (int j0 = h * NH; j0 < j_end; j0 += 32) {
+          // The source sums of item j0 + ((lane + r) & 31) at rotation r: every
+          // lane meets the group's 32 items in turn and hands their sums on.
+          float2 run[6];
+#pragma unroll
+          for (int c = 0; c < 6; ++c) run[c] = make_float2(0.f, 0.f);
 #pragma unroll 2
-        for (int j = h * NH; j < j_end; ++j) {
-          const PairItems::Item it = PairItems::load_item(sp, smv, j);
-          float2 srcf[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-          float2 srcg[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+          for (int r = 0; r < 32; ++r) {
+            const PairItems::Item it = PairItems::load_item(sp, smv, j0 + ((lane + r) & 31));
+            float2 src[6];
 #pragma unroll
-          for (int t = 0; t < TPT; ++t)
-            sym_field_force_pair2(tx[t], ty[t], tz[t], tmx[t], tmy[t], tmz[t], it, nf2, rg, accf[t], accg[t], srcf,
-                                  srcg);
-          if (sym) {  // warp-uniform
-            float v[16];
+            for (int c = 0; c < 6; ++c) src[c] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              v[2 * c] = srcf[c].x;
-              v[2 * c + 1] = srcf[c].y;
-              v[6 + 2 * c] = srcg[c].x;
-              v[6 + 2 * c + 1] = srcg[c].y;
+            for (int t = 0; t < TPT; ++t)
+              sym_field_force_pair2(tx[t], ty[t], tz[t], tmx[t], tmy[t], tmz[t], it, nf2, rg, accf[t], accg[t], src,
+                                    src + 3);
+            if (sym) {  // warp-uniform
+              const int from = (lane + 1) & 31;
+#pragma unroll
+              for (int c = 0; c < 6; ++c) {
+                const float2 v = f2_add(run[c], src[c]);
+                run[c] = make_float2(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from));
+              }
             }
-            v[12] = v[13] = v[14] = v[15] = 0.f;
-            const float w = warp_reduce_scatter<16>(v, lane);
-            const int kv = lane >> 1;
-            if ((lane & 1) == 0 && kv < 12) s_src[wid][(j - h * NH) * kFfRow + kv] = w;
+          }
+          if (sym) {  // back at item `lane`
+            float* d = s_src[wid] + (j0 - h * NH + lane) * kFfRow;
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+              d[2 * c] = run[c].x;
+              d[2 * c + 1] = run[c].y;
+            }
           }
         }
         if (sym) {
