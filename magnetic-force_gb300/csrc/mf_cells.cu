@@ -240,7 +240,7 @@ __global__ void k_gather_sorted(const int32_t* __restrict__ perm, const float4* 
 // them.  Without a branch: pairs beyond the near radius (and a particle with
 // itself, for the force) get zero coefficients.
 struct NearConsts {
-  float near2, h, inv_h, ih3, ih5, ih4k, cA, cB;
+  float near2, h, inv_h, ih3_30, ih5_30, ih4k, cA, cB;
 };
 struct NearTargets {  // two targets: positions, then dipoles (force)
   float4 xy, zm, mm;  // (x0, x1, y0, y1), (z0, z1, mx0, mx1), (my0, my1, mz0, mz1)
@@ -279,7 +279,7 @@ __device__ __forceinline__ void near_pair2(const NearTargets& t, const NearSourc
     const bool in0 = r2.x < c.near2, in1 = r2.y < c.near2;
     float2 al, be;
     field_near_unit2(r2, c.h, c.inv_h, al, be);
-    float2 da = f2_fma(al, f2_dup(c.ih5), f2_dup(-c.cA)), db = f2_fma(be, f2_dup(-c.ih3), f2_dup(c.cB));
+    float2 da = f2_fma(al, f2_dup(c.ih5_30), f2_dup(-c.cA)), db = f2_fma(be, f2_dup(-c.ih3_30), f2_dup(c.cB));
     da = make_float2(in0 ? da.x : 0.f, in1 ? da.y : 0.f);
     db = make_float2(in0 ? db.x : 0.f, in1 ? db.y : 0.f);
     const float2 t3 = f2_mul(f2_mul(ds, f2_dup(3.f)), da);
@@ -346,8 +346,8 @@ __global__ void __launch_bounds__(128) k_correction_cells(const CellGrid* __rest
     nc.near2 = kForce ? g.pc.near2_force : g.pc.near2_field;
     nc.h = g.pc.h;
     nc.inv_h = g.pc.inv_h;
-    nc.ih3 = g.pc.ih3;
-    nc.ih5 = g.pc.ih5;
+    nc.ih3_30 = g.pc.ih3_30;
+    nc.ih5_30 = g.pc.ih5_30;
     nc.ih4k = g.pc.ih4_over_k;
     if (kForce) clamped_force_coeffs(nc.near2, nc.cA, nc.cB);
     else clamped_field_coeffs(nc.near2, nc.cA, nc.cB);
@@ -561,8 +561,8 @@ __global__ void __launch_bounds__(128) k_correction_at(const CellGrid* __restric
         } else {
           float al, be;
           field_near_unit(r2, near_rsqrt(r2), g.pc.h, g.pc.inv_h, al, be);
-          const float t3 = 3.f * ds * fmaf(al, g.pc.ih5, -cA);
-          const float db = fmaf(be, g.pc.ih3, -cB);
+          const float t3 = 3.f * ds * fmaf(al, g.pc.ih5_30, -cA);
+          const float db = fmaf(be, g.pc.ih3_30, -cB);
           acc[0] += dx * t3 - mj.x * db;
           acc[1] += dy * t3 - mj.y * db;
           acc[2] += dz * t3 - mj.z * db;

@@ -37,7 +37,8 @@ struct PairConsts {
   Real inv_h;        // 1/h
   Real h;            // smoothing length
   Real ih3;          // 1/h^3
-  Real ih5;          // 1/h^5
+  Real ih3_30;       // 1/(30 h^3), 1/(30 h^5): scale the field's near forms (field_near_unit)
+  Real ih5_30;
   Real ih4_over_k;   // 1/(h^4 K): scales the fitted curves into the K-free form
   Real near2_field;  // (2h)^2: field pairs closer than this take the SPH branch
   Real near2_force;  // (4h)^2: force pairs at or inside this take the fitted branch
@@ -52,7 +53,8 @@ __host__ __device__ inline PairConsts<Real> make_pair_consts(double h) {
   k.inv_h = Real(1.0 / h);
   k.h = Real(h);
   k.ih3 = Real(1.0 / (h * h * h));
-  k.ih5 = Real(1.0 / (h * h * h * h * h));
+  k.ih3_30 = Real(1.0 / (30.0 * h * h * h));
+  k.ih5_30 = Real(1.0 / (30.0 * h * h * h * h * h));
   k.ih4_over_k = Real(1.0 / (h * h * h * h * kForceK));
   k.near2_field = Real(4.0 * h * h);
   k.near2_force = Real(16.0 * h * h);
@@ -303,35 +305,36 @@ __device__ __forceinline__ void clamped_force_coeffs(float near2, float& P, floa
 // lanes of a warp sit on different pieces.  Same mathematics as
 // field_near_coeffs / force_near_coeffs with the polynomials multiplied out.
 
-// Field: alpha h^5 and beta h^3 at q = r / h < 2.  The outer piece's beta is
-// written in t = 2 - q, where its terms do not cancel (they vanish at q = 2):
-//   q < 1: 0.8 - 0.5 q,                        -8/3 + 4.8 q^2 - 2.5 q^3
-//   else:  q/6 - 0.8 + 1/q - q^-5/15,          2/15 + t/5 + t^2/5 - 5 t^3/6 - q^-3/15
+// Field: 30 alpha h^5 and 30 beta h^3 at q = r / h < 2.  Times 30 every
+// coefficient is a whole number: 0.8f alone would put 4e-7 of alpha at q = 2
+// into every pair.  The outer piece's beta is written in t = 2 - q, where its
+// terms do not cancel.
+//   q < 1: 24 - 15 q,                       -80 + 144 q^2 - 75 q^3
+//   else:  5 q - 24 + 30 / q - 2 q^-5,      4 + 6 t + 6 t^2 - 25 t^3 - 2 q^-3
 // ri: near_rsqrt(r2), finite at r = 0 (where q comes out 0).
 __device__ __forceinline__ float near_rsqrt(float r2) { return rsqrt_approx(fmaxf(r2, 1e-36f)); }
 __device__ __forceinline__ void field_near_unit(float r2, float ri, float h, float inv_h, float& al, float& be) {
   const float q = (r2 * ri) * inv_h, iq = ri * h;
   const float iq2 = iq * iq, iq3 = iq2 * iq, t = 2.f - q;
   const bool hi = q >= 1.f;
-  const float al_hi = fmaf(q, 1.f / 6.f, iq - 0.8f) - (iq3 * iq2) * (1.f / 15.f);
-  const float be_hi = fmaf(t, fmaf(t, fmaf(t, -5.f / 6.f, 0.2f), 0.2f), 2.f / 15.f) - iq3 * (1.f / 15.f);
-  const float al_lo = fmaf(q, -0.5f, 0.8f);
-  const float be_lo = fmaf(q * q, fmaf(q, -2.5f, 4.8f), -8.f / 3.f);
+  const float al_hi = fmaf(iq3 * iq2, -2.f, fmaf(q, 5.f, fmaf(iq, 30.f, -24.f)));
+  const float be_hi = fmaf(iq3, -2.f, fmaf(t, fmaf(t, fmaf(t, -25.f, 6.f), 6.f), 4.f));
+  const float al_lo = fmaf(q, -15.f, 24.f);
+  const float be_lo = fmaf(q * q, fmaf(q, -75.f, 144.f), -80.f);
   al = hi ? al_hi : al_lo;
   be = hi ? be_hi : be_lo;
 }
-
 // The same for two distances at once (packed FP32).
 __device__ __forceinline__ void field_near_unit2(float2 r2, float h, float inv_h, float2& al, float2& be) {
   const float2 ri = make_float2(near_rsqrt(r2.x), near_rsqrt(r2.y));
   const float2 q = f2_mul(f2_mul(r2, ri), f2_dup(inv_h)), iq = f2_mul(ri, f2_dup(h));
   const float2 iq2 = f2_mul(iq, iq), iq3 = f2_mul(iq2, iq), t = f2_sub(f2_dup(2.f), q);
-  const float2 m15 = f2_dup(-1.f / 15.f);
-  const float2 al_hi = f2_fma(f2_mul(iq3, iq2), m15, f2_fma(q, f2_dup(1.f / 6.f), f2_add(iq, f2_dup(-0.8f))));
-  const float2 b3 = f2_fma(t, f2_fma(t, f2_dup(-5.f / 6.f), f2_dup(0.2f)), f2_dup(0.2f));
-  const float2 be_hi = f2_fma(iq3, m15, f2_fma(t, b3, f2_dup(2.f / 15.f)));
-  const float2 al_lo = f2_fma(q, f2_dup(-0.5f), f2_dup(0.8f));
-  const float2 be_lo = f2_fma(f2_mul(q, q), f2_fma(q, f2_dup(-2.5f), f2_dup(4.8f)), f2_dup(-8.f / 3.f));
+  const float2 m2 = f2_dup(-2.f);
+  const float2 al_hi = f2_fma(f2_mul(iq3, iq2), m2, f2_fma(q, f2_dup(5.f), f2_fma(iq, f2_dup(30.f), f2_dup(-24.f))));
+  const float2 b2 = f2_fma(t, f2_fma(t, f2_dup(-25.f), f2_dup(6.f)), f2_dup(6.f));
+  const float2 be_hi = f2_fma(iq3, m2, f2_fma(t, b2, f2_dup(4.f)));
+  const float2 al_lo = f2_fma(q, f2_dup(-15.f), f2_dup(24.f));
+  const float2 be_lo = f2_fma(f2_mul(q, q), f2_fma(q, f2_dup(-75.f), f2_dup(144.f)), f2_dup(-80.f));
   const bool h0 = q.x >= 1.f, h1 = q.y >= 1.f;
   al = make_float2(h0 ? al_hi.x : al_lo.x, h1 ? al_hi.y : al_lo.y);
   be = make_float2(h0 ? be_hi.x : be_lo.x, h1 ? be_hi.y : be_lo.y);
@@ -409,8 +412,8 @@ __device__ __forceinline__ void field_pair_sel(float dx, float dy, float dz, flo
   float al, be;
   field_near_unit(r2, ri, k.h, k.inv_h, al, be);
   const bool far = r2 >= k.near2_field;
-  const float beta = far ? ri3 : be * k.ih3;
-  const float alpha = far ? ri3 * ri2 : al * k.ih5;
+  const float beta = far ? ri3 : be * k.ih3_30;
+  const float alpha = far ? ri3 * ri2 : al * k.ih5_30;
   const float t = (dx * sx + dy * sy + dz * sz) * alpha;
   s1[0] += dx * t;
   s1[1] += dy * t;
