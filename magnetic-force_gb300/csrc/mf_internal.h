@@ -522,6 +522,8 @@ class Fmm {
   mf_status product_q(int kind, const float4* pos4, const float4* smom, const AllPairsArgs<float>& a,
                       const SceneDesc<float>& sc, cudaStream_t st, const double* done, cudaEvent_t* marks,
                       bool sym_near);
+  template <class Far>
+  mf_status build_lists(int L, const std::vector<int64_t>& m, const Far& far, cudaStream_t st);
   FmmConfig cfg_;
   FmmStats stats_;
   int degree_ = 5;
@@ -539,8 +541,8 @@ class Fmm {
   DevBuf tocc_, tcell_of_, tstart_, tcursor_, tperm_tmp_, tperm_;
   bool separate_ = false;
   int64_t nt_ = 0;
+  std::vector<int64_t> lists_key_;  // degree, grid shape and acceptance of the uploaded lists (empty: none)
   std::vector<int4> host_list_, host_rows_, host_hrows_;  // as last uploaded
-  std::vector<int32_t> host_dkey_;           // degree and offsets of the uploaded derivative table
   unsigned long long* hstat_ = nullptr;      // pinned: near pairs, largest leaf, M2L count, occupied leaves, in-box pairs
   cudaEvent_t stat_ev_ = nullptr;
   bool stat_pending_ = false;
@@ -554,8 +556,3 @@ void to_pairs(const float4* src, float4* dst, int64_t n, cudaStream_t st, const 
               int done_total = 0);
 
 }  // namespace mfgb
-
-// Element-wise equality of CUDA's int4 (host-side comparison of uploaded tables).
-inline bool operator==(const int4& a, const int4& b) { return a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w; }
-inline bool operator!=(const int4& a, const int4& b) { return !(a == b); }
-
