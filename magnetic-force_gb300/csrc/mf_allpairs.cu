@@ -233,6 +233,10 @@ template <>
 struct BodyOf<float, Body::ForceF2> {
   using type = ForceF2Body;
 };
+template <>
+struct BodyOf<float, Body::TensorF2> {
+  using type = TensorF2Body;
+};
 
 // Packed two-source bodies exist in FP32 only.
 template <class Real>
@@ -242,7 +246,7 @@ constexpr bool has_f2() {
 
 // Launch configuration: FP32 shaped bodies take shape S of kShapeTable;
 // the tensor body and FP64 keep KCfg (shape 0 only).
-template <class Real, Body B, int S, bool kShaped = std::is_same<Real, float>::value && B != Body::Tensor>
+template <class Real, Body B, int S, bool kShaped = std::is_same<Real, float>::value && shaped(B)>
 struct LCfg : KCfg<Real, B> {};
 template <class Real, Body B, int S>
 struct LCfg<Real, B, S, true> {
@@ -325,6 +329,10 @@ static void cfg_of(Body b, int* tile, int* tbt, int shape) {
       *tile = KCfg<float, Body::ForceF2>::TILE;
       *tbt = KCfg<float, Body::ForceF2>::TPB * KCfg<float, Body::ForceF2>::TPT;
       break;
+    case Body::TensorF2:
+      *tile = KCfg<float, Body::TensorF2>::TILE;
+      *tbt = KCfg<float, Body::TensorF2>::TPB * KCfg<float, Body::TensorF2>::TPT;
+      break;
   }
 }
 
@@ -397,7 +405,7 @@ mf_status refresh_plan_coefs(const std::vector<SceneSpec>& specs, Plan<Real>& pl
 template <class Real, Body B>
 struct Shaped {
   static void needs(const Plan<Real>& plan, size_t* pd, size_t* nc) {
-    if constexpr (std::is_same<Real, float>::value && B != Body::Tensor) {
+    if constexpr (std::is_same<Real, float>::value && shaped(B)) {
       switch (plan.shape) {
         case 1: return Launcher<Real, B, 1>::needs(plan, pd, nc);
         case 2: return Launcher<Real, B, 2>::needs(plan, pd, nc);
@@ -410,7 +418,7 @@ struct Shaped {
   }
   static mf_status launch(const Plan<Real>& plan, const LaunchIO<Real>& io, double* partials, int32_t* counters,
                           int32_t* err, cudaStream_t st) {
-    if constexpr (std::is_same<Real, float>::value && B != Body::Tensor) {
+    if constexpr (std::is_same<Real, float>::value && shaped(B)) {
       switch (plan.shape) {
         case 1: return Launcher<Real, B, 1>::launch(plan, io, partials, counters, err, st);
         case 2: return Launcher<Real, B, 2>::launch(plan, io, partials, counters, err, st);
@@ -441,6 +449,9 @@ void plan_scratch_needs(const Plan<Real>& plan, size_t* pd, size_t* nc) {
     case Body::ForceF2:
       if constexpr (has_f2<Real>()) Shaped<float, Body::ForceF2>::needs(plan, pd, nc);
       break;
+    case Body::TensorF2:
+      if constexpr (has_f2<Real>()) Shaped<float, Body::TensorF2>::needs(plan, pd, nc);
+      break;
   }
 }
 
@@ -460,6 +471,9 @@ mf_status run_plan_raw(const Plan<Real>& plan, const LaunchIO<Real>& io, double*
       break;
     case Body::ForceF2:
       if constexpr (has_f2<Real>()) return Shaped<float, Body::ForceF2>::launch(plan, io, partials, counters, err, st);
+      break;
+    case Body::TensorF2:
+      if constexpr (has_f2<Real>()) return Shaped<float, Body::TensorF2>::launch(plan, io, partials, counters, err, st);
       break;
   }
   return fail(MF_ERR_UNSUPPORTED, "packed two-source kernels exist in FP32 only");
@@ -504,6 +518,7 @@ const char* body_name(Body b) {
     case Body::Tensor: return "tensor";
     case Body::FieldF2: return "field_packed";
     case Body::ForceF2: return "force_packed";
+    case Body::TensorF2: return "tensor_packed";
   }
   return "?";
 }

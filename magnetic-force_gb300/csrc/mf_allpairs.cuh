@@ -399,19 +399,19 @@ struct ForceF2Body : PairItems {
   }
 };
 
-// Packed force tensor (the FMM matrix of the Hessian kernel at separate
-// targets).  The near-field correction comes as two records per target in
-// corr4: (xx, yy, zz, -), (xy, xz, yz, -).
+// Packed force tensor (direct sums and the FMM matrix of the Hessian kernel).
+// The near-field correction comes as two records per target in corr4: (xx, yy,
+// zz, -), (xy, xz, yz, -).
 struct TensorF2Body : PairItems {
   static constexpr int kOut = 6;
   struct TData {
     float2 x, y, z;
   };
   struct Acc {
-    float2 t[6];
+    float2 t[7];
     __device__ void zero() {
 #pragma unroll
-      for (int k = 0; k < 6; ++k) t[k] = make_float2(0.f, 0.f);
+      for (int k = 0; k < 7; ++k) t[k] = make_float2(0.f, 0.f);
     }
   };
   __device__ static void load(const AllPairsArgs<float>& a, int64_t i, TData& t) {
@@ -425,8 +425,12 @@ struct TensorF2Body : PairItems {
   }
   __device__ static void tile_out(const Acc& acc, float* o) {
     const float c = float(kForceK);
+    const float tr = acc.t[6].x + acc.t[6].y;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) o[k] = (acc.t[k].x + acc.t[k].y) * c;
+    for (int k = 0; k < 3; ++k) {
+      o[k] = fmaf(2.f, acc.t[3 + k].x + acc.t[3 + k].y, tr) * c;
+      o[3 + k] = (acc.t[k].x + acc.t[k].y) * c;
+    }
   }
   __device__ static void epilogue(const AllPairsArgs<float>& a, const SceneDesc<float>& sc, int64_t i,
                                   const TData&, const double* vin) {

@@ -39,7 +39,15 @@ unsigned grid_for(int64_t n) {
   return unsigned(g);
 }
 
-constexpr int kBodies = 5;
+constexpr int kBodies = 6;
+
+// Target-source pairs from which the packed kernels beat the exact-branch
+// ones.  They need a cell list (ten launches, a host round trip) and the
+// near-field correction: whole calls at 4,000 x 4,000, 10,000 x 10,000 and
+// 12,000 x 12,000 take 176 / 264 / 303 us packed and 100 / 237 / 313 exact
+// for the field, 227 / 401 / 464 and 124 / 374 / 460 for the tensor, 217 /
+// 375 / 421 and 126 / 341 / 470 for the force.
+constexpr double kPackedDirectMin = 1.25e8;
 
 struct DirectCtx {
   std::mutex mu;
@@ -118,14 +126,14 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
   io.tpos = c.t4.as<float4>();
   io.spos = c.s4.as<float4>();
   io.smom = c.m4.as<float4>();
-  // Field and force go through the packed two-source kernels: sources in pair
+  // Large calls go through the packed two-source kernels: sources in pair
   // layout, a cell list over the sources, and the near-field correction.
   Body launch_body = body;
-  if (body == Body::Field || body == Body::Force) {
+  if (double(nt) * double(ns) >= kPackedDirectMin) {
     const size_t pair_bytes = size_t(ns + 1) * sizeof(float4);
     MF_TRY(c.s2.reserve(pair_bytes));
     MF_TRY(c.m2.reserve(pair_bytes));
-    MF_TRY(c.corr.reserve(size_t(nt) * sizeof(float4)));
+    MF_TRY(c.corr.reserve(size_t(nt) * (body == Body::Tensor ? 2 : 1) * sizeof(float4)));
     to_pairs(c.s4.as<float4>(), c.s2.as<float4>(), ns, st);
     to_pairs(c.m4.as<float4>(), c.m2.as<float4>(), ns, st);
     MF_CUDA_TRY(cudaGetLastError());
@@ -137,6 +145,10 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
         MF_TRY(c.cells.field_correction_at(c.t4.as<float4>(), nt, c.s4.as<float4>(), c.m4.as<float4>(),
                                            c.corr.as<float4>(), st));
       launch_body = Body::FieldF2;
+    } else if (body == Body::Tensor) {
+      MF_TRY(c.cells.tensor_correction_at(c.t4.as<float4>(), nt, c.s4.as<float4>(), c.m4.as<float4>(),
+                                          c.corr.as<float4>(), st));
+      launch_body = Body::TensorF2;
     } else {
       MF_TRY(c.cells.force_correction(c.s4.as<float4>(), c.m4.as<float4>(), c.corr.as<float4>(), st));
       launch_body = Body::ForceF2;

@@ -95,24 +95,26 @@ struct DevBuf {
 // All-pairs launch configurations.
 // ---------------------------------------------------------------------------
 // Field / Force / Tensor: one packed record per source, exact pair branches
-// (both precisions).  FieldF2 / ForceF2: FP32 pair-layout sources, two
-// sources per instruction, clamped far form plus a near-field correction
+// (both precisions).  FieldF2 / ForceF2 / TensorF2: FP32 pair-layout sources,
+// two sources per instruction, clamped far form plus a near-field correction
 // array (mf_cells.cu) added in the epilogue.
-enum class Body { Field = 0, Force = 1, Tensor = 2, FieldF2 = 3, ForceF2 = 4 };
+enum class Body { Field = 0, Force = 1, Tensor = 2, FieldF2 = 3, ForceF2 = 4, TensorF2 = 5 };
 
 // Scene sizes from which the packed path (clamped far form + near-field
 // correction) beats the exact-branch kernels.  Near pairs per particle are
 // fixed by the density (~270 inside 2h, ~2100 inside 4h at h = 2 spacings)
 // while far pairs grow with N, and a corrected near pair costs several far
 // pairs, so small scenes stay on the exact-branch kernels.
-// Force, one scene alone: 0.43 ms exact against 0.51 ms packed at 12,288
-// particles, 0.70 against 0.66 at 16,384.
+// Force, one scene alone (whole steps, exact against packed): 404 / 449 us at
+// 6,000 particles, 519 / 523 at 8,000, 638 / 605 at 10,000, 756 / 699 at
+// 12,289.  (Before the correction took two targets per instruction the line
+// lay at 14,336.)
 constexpr int64_t kPackedFieldMin = 2048;
-constexpr int64_t kPackedForceMin = 14336;
+constexpr int64_t kPackedForceMin = 8192;
 // Force inside a batch: one packed launch and one correction launch serve all
 // large scenes, so the packed path wins from smaller scenes on (256 scenes of
-// 512..32,768 particles: 92.2 ms per step at 12,288, 89.7 ms at 4,096, flat
-// below).
+// 512..32,768 particles: 92.2 ms per step at 12,288, 89.7 ms at 4,096; 64 of
+// 512..4,096: 8.5 ms per four steps at 4,096, 9.1 at 2,048).
 constexpr int64_t kBatchPackedForceMin = 4096;
 // Direct entries (no tuning): the packed products once per unordered pair
 // from this size on.  Measured against the best all-pairs shape at 32,768
@@ -150,6 +152,10 @@ template <>
 struct KCfg<float, Body::ForceF2> {
   static constexpr int TPB = 256, TPT = 2, TILE = 256, STAGES = 3, kOut = 4;
 };
+template <>
+struct KCfg<float, Body::TensorF2> {
+  static constexpr int TPB = 128, TPT = 2, TILE = 256, STAGES = 3, kOut = 6;
+};
 // FP64: 128 threads x 1 target, 128-source tiles of 32-byte records.
 template <>
 struct KCfg<double, Body::Field> {
@@ -173,7 +179,7 @@ struct Shape {
 };
 constexpr int kShapes = 5;
 constexpr Shape kShapeTable[kShapes] = {{256, 2, 256}, {128, 2, 256}, {256, 1, 256}, {128, 4, 128}, {128, 4, 256}};
-inline bool shaped(Body b) { return b != Body::Tensor; }
+constexpr bool shaped(Body b) { return b != Body::Tensor && b != Body::TensorF2; }
 // Shape index of the products evaluated once per unordered pair, for scenes
 // whose targets are their sources: the packed FP32 field / force
 // (mf_sympair.cu) and the FP64 ones (mf_sym64.cu).

@@ -264,8 +264,12 @@ __device__ __forceinline__ void force_pair2(float2 tx, float2 ty, float2 tz, flo
   f[2] = f2_fma(dz, w, f2_fma(smz, v, f[2]));
 }
 
-// Packed two-source force tensor (6 unique entries xx, yy, zz, xy, xz, yz of
-// T(d, s) / K), clamped far form: P = r^-5, Q = -5 r^-7 at max(r^2, near2).
+// Packed two-source force tensor, clamped far form: with e = P d and
+// v = m - 5/2 r^-2 (d.m) d,
+//   T / K = e v^T + v e^T + P (d.m) I,
+// summed as the off-diagonal entries t[0..2] (xy, xz, yz), half the diagonal
+// ones without the trace term t[3..5], and the trace term t[6]: 30 packed
+// operations (entry by entry 46).
 __device__ __forceinline__ void tensor_pair2(float2 tx, float2 ty, float2 tz, float2 sx, float2 sy, float2 sz,
                                              float2 smx, float2 smy, float2 smz, float near2, float2* t) {
   const float2 dx = f2_sub(tx, sx), dy = f2_sub(ty, sy), dz = f2_sub(tz, sz);
@@ -273,17 +277,17 @@ __device__ __forceinline__ void tensor_pair2(float2 tx, float2 ty, float2 tz, fl
   const float2 ri = clamp_rsqrt2(r2, near2);
   const float2 ri2 = f2_mul(ri, ri);
   const float2 P = f2_mul(f2_mul(ri2, ri2), ri);
-  const float2 Q = f2_mul(f2_mul(ri2, P), f2_dup(-5.f));
   const float2 ds = f2_fma(dz, smz, f2_fma(dy, smy, f2_mul(dx, smx)));
-  const float2 pd = f2_mul(P, ds), qd = f2_mul(Q, ds);
-  const float2 ax = f2_mul(P, smx), ay = f2_mul(P, smy), az = f2_mul(P, smz);
-  const float2 two = f2_dup(2.f);
-  t[0] = f2_fma(f2_mul(qd, dx), dx, f2_fma(f2_mul(two, ax), dx, f2_add(pd, t[0])));
-  t[1] = f2_fma(f2_mul(qd, dy), dy, f2_fma(f2_mul(two, ay), dy, f2_add(pd, t[1])));
-  t[2] = f2_fma(f2_mul(qd, dz), dz, f2_fma(f2_mul(two, az), dz, f2_add(pd, t[2])));
-  t[3] = f2_fma(f2_mul(qd, dx), dy, f2_fma(ax, dy, f2_fma(ay, dx, t[3])));
-  t[4] = f2_fma(f2_mul(qd, dx), dz, f2_fma(ax, dz, f2_fma(az, dx, t[4])));
-  t[5] = f2_fma(f2_mul(qd, dy), dz, f2_fma(ay, dz, f2_fma(az, dy, t[5])));
+  const float2 k = f2_mul(f2_mul(ri2, f2_dup(-2.5f)), ds);
+  const float2 vx = f2_fma(dx, k, smx), vy = f2_fma(dy, k, smy), vz = f2_fma(dz, k, smz);
+  const float2 ex = f2_mul(dx, P), ey = f2_mul(dy, P), ez = f2_mul(dz, P);
+  t[0] = f2_fma(ex, vy, f2_fma(ey, vx, t[0]));
+  t[1] = f2_fma(ex, vz, f2_fma(ez, vx, t[1]));
+  t[2] = f2_fma(ey, vz, f2_fma(ez, vy, t[2]));
+  t[3] = f2_fma(ex, vx, t[3]);
+  t[4] = f2_fma(ey, vy, t[4]);
+  t[5] = f2_fma(ez, vz, t[5]);
+  t[6] = f2_fma(P, ds, t[6]);
 }
 
 // The clamped far coefficients every near pair received in the packed loop
@@ -441,13 +445,24 @@ __device__ __forceinline__ void force_pair_sel(float dx, float dy, float dz, flo
   f[2] += dz * w + mz * u + sz * v;
 }
 
+// (P, Q) of the force tensor for any pair, FP32 without a branch (k.tbl set).
+__device__ __forceinline__ void force_coeffs_sel(float r2, const PairConsts<float>& k, float& P, float& Q) {
+  float Pn, Qn;
+  force_near_pq(r2, k.tbl, k.inv_h, k.ih4_over_k, Pn, Qn);
+  const float ri = rsqrt_approx(r2), ri2 = ri * ri, ri5 = ri2 * ri2 * ri;
+  const bool far = r2 > k.near2_force, apart = r2 > 0.f;
+  P = far ? ri5 : apart ? Pn : 0.f;
+  Q = far ? -5.f * ri5 * ri2 : apart ? Qn : 0.f;
+}
+
 // One tensor pair (6 unique entries xx, yy, zz, xy, xz, yz): t += T(d, s) / K.
 template <class Real>
 __device__ __forceinline__ void tensor_pair(Real dx, Real dy, Real dz, Real sx, Real sy, Real sz,
                                             const PairConsts<Real>& k, Real* t) {
   Real r2 = dx * dx + dy * dy + dz * dz;
   Real P, Q;
-  force_coeffs(r2, k, P, Q);
+  if constexpr (sizeof(Real) == 4) force_coeffs_sel(r2, k, P, Q);
+  else force_coeffs(r2, k, P, Q);
   Real ds = dx * sx + dy * sy + dz * sz;
   Real pd = P * ds, qd = Q * ds;
   Real ax = P * sx, ay = P * sy, az = P * sz;
