@@ -219,14 +219,29 @@ __global__ void k_sort_cells(const int32_t* __restrict__ start, int64_t n_cells,
   }
 }
 
+// Records 2 p and 2 p + 1 of src[0..n) in pair layout (a missing partner as zeros).
+__device__ __forceinline__ void pair_records(const float4* __restrict__ src, float4* __restrict__ dst, int64_t n,
+                                             int64_t p) {
+  const float4 a = src[2 * p];
+  const float4 b = (2 * p + 1 < n) ? src[2 * p + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+  dst[2 * p] = make_float4(a.x, b.x, a.y, b.y);
+  dst[2 * p + 1] = make_float4(a.z, b.z, 0.f, 0.f);
+}
+
 __constant__ ForceTable c_fit_tbl = make_force_table();
 
 // The binned particles in cell order (positions and the product's dipoles),
-// so the correction reads each row of cells as one contiguous range.
+// so the correction reads each row of cells as one contiguous range.  mom2
+// (optional): the dipoles mom[0..n) in pair layout too (to_pairs), for the
+// packed product that follows.
 __global__ void k_gather_sorted(const int32_t* __restrict__ perm, const float4* __restrict__ pos,
                                 const float4* __restrict__ mom, int64_t n, float4* __restrict__ spos,
-                                float4* __restrict__ smom, const int32_t* __restrict__ done_count, int done_total) {
+                                float4* __restrict__ smom, const int32_t* __restrict__ done_count, int done_total,
+                                float4* __restrict__ mom2) {
   if (done_count && *done_count >= done_total) return;
+  if (mom2)
+    for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < (n + 1) / 2; p += int64_t(gridDim.x) * blockDim.x)
+      pair_records(mom, mom2, n, p);
   for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += int64_t(gridDim.x) * blockDim.x) {
     const int32_t i = perm[q];
     spos[q] = pos[i];
@@ -592,12 +607,8 @@ __global__ void k_to_pairs(const float4* __restrict__ src, float4* __restrict__ 
                            const int32_t* __restrict__ done_count, int done_total) {
   if (done_count && *done_count >= done_total) return;
   const int64_t np = (n + 1) / 2;
-  for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < np; p += int64_t(gridDim.x) * blockDim.x) {
-    const float4 a = src[2 * p];
-    const float4 b = (2 * p + 1 < n) ? src[2 * p + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
-    dst[2 * p] = make_float4(a.x, b.x, a.y, b.y);
-    dst[2 * p + 1] = make_float4(a.z, b.z, 0.f, 0.f);
-  }
+  for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < np; p += int64_t(gridDim.x) * blockDim.x)
+    pair_records(src, dst, n, p);
 }
 
 unsigned grid_for(int64_t n, int per_block = 256) {
@@ -736,9 +747,9 @@ static unsigned cell_grid(int64_t cells) {
 
 mf_status CellList::field_correction(const float4* pos4, const float4* mom4, float4* corr, cudaStream_t st,
                                      const double* done_flags, int done_stride, const int32_t* done_count,
-                                     int done_total) const {
+                                     int done_total, float4* mom2) const {
   k_gather_sorted<<<grid_for(n_total_), 256, 0, st>>>(perm_.as<int32_t>(), pos4, mom4, n_total_, spos_.as<float4>(),
-                                                      smom_.as<float4>(), done_count, done_total);
+                                                      smom_.as<float4>(), done_count, done_total, mom2);
   auto* k = n_cells_ < kSplitCells ? k_correction_cells<false, 4> : k_correction_cells<false, 1>;
   k<<<cell_grid(n_cells_ < kSplitCells ? n_cells_ : (n_cells_ + 3) / 4), 128, 0, st>>>(
       grids_.as<CellGrid>(), n_scenes_, n_cells_, perm_.as<int32_t>(), cell_start_.as<int32_t>(), spos_.as<float4>(),
@@ -762,7 +773,7 @@ mf_status CellList::correction_at(const float4* tpos4, int64_t nt, const float4*
                                   float4* corr, cudaStream_t st) const {
   if (n_scenes_ != 1) return fail(MF_ERR_INVALID_ARG, "separate targets need a single-scene cell list");
   k_gather_sorted<<<grid_for(n_total_), 256, 0, st>>>(perm_.as<int32_t>(), pos4, mom4, n_total_, spos_.as<float4>(),
-                                                      smom_.as<float4>(), nullptr, 0);
+                                                      smom_.as<float4>(), nullptr, 0, nullptr);
   k_correction_at<kTensor><<<cell_grid((nt + 3) / 4), 128, 0, st>>>(
       grids_.as<CellGrid>(), nt, cell_start_.as<int32_t>(), spos_.as<float4>(), smom_.as<float4>(), tpos4, corr);
   MF_CUDA_TRY(cudaGetLastError());
@@ -787,9 +798,10 @@ mf_status CellList::set_skips(const std::vector<int32_t>& field, const std::vect
   return MF_OK;
 }
 
-mf_status CellList::force_correction(const float4* pos4, const float4* mom4, float4* corr, cudaStream_t st) const {
+mf_status CellList::force_correction(const float4* pos4, const float4* mom4, float4* corr, cudaStream_t st,
+                                     float4* mom2) const {
   k_gather_sorted<<<grid_for(n_total_), 256, 0, st>>>(perm_.as<int32_t>(), pos4, mom4, n_total_, spos_.as<float4>(),
-                                                      smom_.as<float4>(), nullptr, 0);
+                                                      smom_.as<float4>(), nullptr, 0, mom2);
   k_correction_cells<true, 4><<<cell_grid(n_cells_), 128, 0, st>>>(
       grids_.as<CellGrid>(), n_scenes_, n_cells_, perm_.as<int32_t>(), cell_start_.as<int32_t>(), spos_.as<float4>(),
       smom_.as<float4>(), corr, skip_force_on_ ? skip_force_.as<int32_t>() : nullptr, nullptr, 0, nullptr, 0);

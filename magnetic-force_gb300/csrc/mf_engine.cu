@@ -419,21 +419,24 @@ class Engine final : public EngineBase {
     if (layout != MF_LAYOUT_AOS && layout != MF_LAYOUT_SOA) return fail(MF_ERR_INVALID_ARG, "bad layout");
     if (where != MF_HOST && where != MF_DEVICE) return fail(MF_ERR_INVALID_ARG, "bad memory kind");
     const int64_t n = np_;
-    // Gather the three SoA components into a device staging buffer first.
     const size_t esz = f64 ? sizeof(double) : sizeof(float);
     MF_TRY(staging_.reserve(size_t(3 * n) * sizeof(double)));
-    MF_TRY(staging2_.reserve(size_t(3 * n) * sizeof(double)));
-    char* soa = staging2_.template as<char>();
-    for (int k = 0; k < 3; ++k) MF_TRY(component_to(q, k, soa + size_t(k * n) * esz, f64));
-    void* dev_out = staging_.ptr;
-    if (layout == MF_LAYOUT_SOA) {
-      dev_out = soa;
-    } else {
-      // SoA -> AoS on the device.
-      if (f64)
-        MF_TRY(soa_to_aos<double>(reinterpret_cast<const double*>(soa), staging_.template as<double>(), n));
-      else
-        MF_TRY(soa_to_aos<float>(reinterpret_cast<const float*>(soa), staging_.template as<float>(), n));
+    // The published arrays are x, y, z one after another.  Where their type is
+    // the one asked for and the result is written elsewhere first (AoS) or goes
+    // to the host, they are read in place: a device destination may be one of
+    // these arrays itself.  Else the components are gathered.
+    const void* soa = layout == MF_LAYOUT_AOS || where == MF_HOST ? published_soa(q, f64) : nullptr;
+    if (!soa) {
+      MF_TRY(staging2_.reserve(size_t(3 * n) * sizeof(double)));
+      char* parts = staging2_.template as<char>();
+      for (int k = 0; k < 3; ++k) MF_TRY(component_to(q, k, parts + size_t(k * n) * esz, f64));
+      soa = parts;
+    }
+    const void* dev_out = soa;
+    if (layout == MF_LAYOUT_AOS) {  // SoA -> AoS on the device
+      if (f64) MF_TRY(soa_to_aos<double>(static_cast<const double*>(soa), staging_.template as<double>(), n));
+      else MF_TRY(soa_to_aos<float>(static_cast<const float*>(soa), staging_.template as<float>(), n));
+      dev_out = staging_.ptr;
     }
     const size_t bytes = size_t(3 * n) * esz;
     MF_CUDA_TRY(cudaMemcpyAsync(dst, dev_out, bytes,
@@ -942,10 +945,9 @@ class Engine final : public EngineBase {
   mf_status prepare_packed(const R4* src_mom, bool force, LaunchIO<Real>& io) {
     if constexpr (kF32) {
       MF_TRY(ensure_cells());
-      to_pairs(src_mom, mom2_.template as<float4>(), np_, st_);
-      MF_CUDA_TRY(cudaGetLastError());
-      if (force) MF_TRY(cells_.force_correction(pos4(), src_mom, corr_.template as<float4>(), st_));
-      else MF_TRY(cells_.field_correction(pos4(), src_mom, corr_.template as<float4>(), st_));
+      float4* m2 = mom2_.template as<float4>();
+      if (force) MF_TRY(cells_.force_correction(pos4(), src_mom, corr_.template as<float4>(), st_, m2));
+      else MF_TRY(cells_.field_correction(pos4(), src_mom, corr_.template as<float4>(), st_, nullptr, 0, nullptr, 0, m2));
       ctr_.kernel_launches += 2;
       io.spos = pos2_.template as<float4>();
       io.smom = mom2_.template as<float4>();
@@ -1389,6 +1391,14 @@ class Engine final : public EngineBase {
 
   template <class T>
   mf_status soa_to_aos(const T* soa, T* aos, int64_t n);
+
+  // Quantity q's published x, y, z arrays (3 n values in a row) in the asked
+  // type, or null where they have to be gathered or converted.
+  const void* published_soa(int q, bool f64) const {
+    if (q == MF_Q_VELOCITY) return nullptr;
+    if (!f64) return pubf(q, 0);
+    return !kF32 && q != MF_Q_POSITIONS ? static_cast<const void*>(pubr(q, 0)) : nullptr;
+  }
 
   // Component k of quantity q into dst (device), as float or double.
   mf_status component_to(int q, int k, void* dst, bool f64) {

@@ -395,11 +395,14 @@ class CellList {
   // clamped far term the packed all-pairs loop gave that pair], in the
   // all-pairs kernels' output units.  Targets = sources = the binned set.
   // done_flags (per-scene solver rows) skip stopped scenes; done_count /
-  // done_total make the launch a no-op once every scene has stopped.
+  // done_total make the launch a no-op once every scene has stopped.  mom2
+  // (single-scene lists over particles 0..n): the dipoles in pair layout as
+  // well, written by the same launch that sorts them.
   mf_status field_correction(const float4* pos4, const float4* mom4, float4* corr, cudaStream_t st,
                              const double* done_flags = nullptr, int done_stride = 0,
-                             const int32_t* done_count = nullptr, int done_total = 0) const;
-  mf_status force_correction(const float4* pos4, const float4* mom4, float4* corr, cudaStream_t st) const;
+                             const int32_t* done_count = nullptr, int done_total = 0, float4* mom2 = nullptr) const;
+  mf_status force_correction(const float4* pos4, const float4* mom4, float4* corr, cudaStream_t st,
+                             float4* mom2 = nullptr) const;
   // Scenes (by build order) whose field / force use the exact-branch kernels
   // and so need no correction.
   mf_status set_skips(const std::vector<int32_t>& field, const std::vector<int32_t>& force);
