@@ -657,6 +657,66 @@ __device__ __forceinline__ int near_plane(const int4& hr, int dx) {
   return 1 + hr.w + ((hr.y == 0 && hr.z == 0) ? dx - 1 : dx + hr.x);
 }
 
+// w^k / k! for k < Q, `stride` apart.
+template <int Q>
+__device__ __forceinline__ void power_table(float w, float* pw, int stride) {
+  float v = 1.f;
+  pw[0] = 1.f;
+#pragma unroll
+  for (int k = 1; k < Q; ++k) {
+    v = v * w * (1.f / float(k));
+    pw[k * stride] = v;
+  }
+}
+
+// The local expansion's terms g = g0, g0 + gstep, ...: h = sum_g L_(g + e_k)
+// w^g / g! (kKind 0, x y z) or sum_g L_(g + e_a + e_b) w^g / g! (xx, yy, zz, xy,
+// xz, yz).  pw: the target's columns of the three power tables.
+template <int Q, int kKind>
+__device__ __forceinline__ void local_terms(const float* pw, int stride, const float* s_L, int g0, int gstep, float* h) {
+#pragma unroll
+  for (int q = 0; q < 6; ++q) h[q] = 0.f;
+  for (int g = g0; g < ncoef(kKind == 0 ? Q - 1 : Q - 2); g += gstep) {
+    const char4 e = c_mi.v[g];
+    const float mono = pw[e.x * stride] * pw[(Q + e.y) * stride] * pw[(2 * Q + e.z) * stride];
+    if constexpr (kKind == 0) {
+      h[0] = fmaf(s_L[gidx(e.x + 1, e.y, e.z) - 1], mono, h[0]);
+      h[1] = fmaf(s_L[gidx(e.x, e.y + 1, e.z) - 1], mono, h[1]);
+      h[2] = fmaf(s_L[gidx(e.x, e.y, e.z + 1) - 1], mono, h[2]);
+    } else {
+      h[0] = fmaf(s_L[gidx(e.x + 2, e.y, e.z) - 1], mono, h[0]);
+      h[1] = fmaf(s_L[gidx(e.x, e.y + 2, e.z) - 1], mono, h[1]);
+      h[2] = fmaf(s_L[gidx(e.x, e.y, e.z + 2) - 1], mono, h[2]);
+      h[3] = fmaf(s_L[gidx(e.x + 1, e.y + 1, e.z) - 1], mono, h[3]);
+      h[4] = fmaf(s_L[gidx(e.x + 1, e.y, e.z + 1) - 1], mono, h[4]);
+      h[5] = fmaf(s_L[gidx(e.x, e.y + 1, e.z + 1) - 1], mono, h[5]);
+    }
+  }
+}
+
+// The far field from these sums: H = -grad phi = -h / (4 pi s^3); Hess phi =
+// h / (4 pi s^4), F = -mu0 Hess phi m_t, the tensor -mu0 Hess phi.
+template <int kKind>
+__device__ __forceinline__ void add_far(const float* h, float inv_s, const AllPairsArgs<float>& a, int64_t i, double* v) {
+  if constexpr (kKind == 0) {
+    const double f = -kInv4Pi * double(inv_s) * double(inv_s) * double(inv_s);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) v[q] += f * double(h[q]);
+  } else {
+    const double is2 = double(inv_s) * double(inv_s);
+    const double f = -kMu0 * kInv4Pi * is2 * is2;
+    if constexpr (kKind == 1) {
+      const float4 tm = a.tmom[i];
+      v[0] += f * (double(h[0]) * tm.x + double(h[3]) * tm.y + double(h[4]) * tm.z);
+      v[1] += f * (double(h[3]) * tm.x + double(h[1]) * tm.y + double(h[5]) * tm.z);
+      v[2] += f * (double(h[4]) * tm.x + double(h[5]) * tm.y + double(h[2]) * tm.z);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 6; ++q) v[q] += f * double(h[q]);
+    }
+  }
+}
+
 // kKind: 0 field (H), 1 Kelvin force (contracted with the target dipole),
 // 2 force tensor (the Hessian kernel's 3x3 at each target).
 // kParts (force, targets = sources): the near field is not swept here but
@@ -819,63 +879,12 @@ __global__ void __launch_bounds__(TPB) k_fmm_p2p(const P2PArgs p, const AllPairs
                         (tp.y - (lv.oy + (float(iy) + 0.5f) * lv.side)) * inv_s,
                         (tp.z - (lv.oz + (float(iz) + 0.5f) * lv.side)) * inv_s};
 #pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-      float v = 1.f;
-      pw[(ax * Q) * TPB + tid] = 1.f;
-#pragma unroll
-      for (int k = 1; k < Q; ++k) {
-        v = v * w[ax] * (1.f / float(k));
-        pw[(ax * Q + k) * TPB + tid] = v;
-      }
-    }
+    for (int ax = 0; ax < 3; ++ax) power_table<Q>(w[ax], pw + ax * Q * TPB + tid, TPB);
     double v[kOut];
     for (int q = 0; q < kOut; ++q) v[q] = double(run[q]) + double(cmp[q]);
-    if constexpr (kKind == 0) {
-      // H = -grad phi = -1/(4 pi s^3) sum_g L_(g + e_k) w^g / g!
-      float h0 = 0.f, h1 = 0.f, h2 = 0.f;
-      for (int g = 0; g < ncoef(Q - 1); ++g) {
-        const char4 e = c_mi.v[g];
-        const float mono = pw[e.x * TPB + tid] * pw[(Q + e.y) * TPB + tid] *
-                           pw[(2 * Q + e.z) * TPB + tid];
-        h0 = fmaf(s_L[gidx(e.x + 1, e.y, e.z) - 1], mono, h0);
-        h1 = fmaf(s_L[gidx(e.x, e.y + 1, e.z) - 1], mono, h1);
-        h2 = fmaf(s_L[gidx(e.x, e.y, e.z + 1) - 1], mono, h2);
-      }
-      const double f = -kInv4Pi * double(inv_s) * double(inv_s) * double(inv_s);
-      v[0] += f * double(h0);
-      v[1] += f * double(h1);
-      v[2] += f * double(h2);
-    } else {
-      // Hess phi = 1/(4 pi s^4) sum_g L_(g + e_a + e_b) w^g / g!;  F = -mu0 Hess phi m_t
-      float hxx = 0.f, hyy = 0.f, hzz = 0.f, hxy = 0.f, hxz = 0.f, hyz = 0.f;
-      for (int g = 0; g < ncoef(Q - 2); ++g) {
-        const char4 e = c_mi.v[g];
-        const float mono = pw[e.x * TPB + tid] * pw[(Q + e.y) * TPB + tid] *
-                           pw[(2 * Q + e.z) * TPB + tid];
-        hxx = fmaf(s_L[gidx(e.x + 2, e.y, e.z) - 1], mono, hxx);
-        hyy = fmaf(s_L[gidx(e.x, e.y + 2, e.z) - 1], mono, hyy);
-        hzz = fmaf(s_L[gidx(e.x, e.y, e.z + 2) - 1], mono, hzz);
-        hxy = fmaf(s_L[gidx(e.x + 1, e.y + 1, e.z) - 1], mono, hxy);
-        hxz = fmaf(s_L[gidx(e.x + 1, e.y, e.z + 1) - 1], mono, hxz);
-        hyz = fmaf(s_L[gidx(e.x, e.y + 1, e.z + 1) - 1], mono, hyz);
-      }
-      const double is2 = double(inv_s) * double(inv_s);
-      const double f = -kMu0 * kInv4Pi * is2 * is2;
-      if constexpr (kForce) {
-        const float4 tm = a.tmom[i];
-        v[0] += f * (double(hxx) * tm.x + double(hxy) * tm.y + double(hxz) * tm.z);
-        v[1] += f * (double(hxy) * tm.x + double(hyy) * tm.y + double(hyz) * tm.z);
-        v[2] += f * (double(hxz) * tm.x + double(hyz) * tm.y + double(hzz) * tm.z);
-      } else {
-        // T = -mu0 Hess phi, entries xx, yy, zz, xy, xz, yz
-        v[0] += f * double(hxx);
-        v[1] += f * double(hyy);
-        v[2] += f * double(hzz);
-        v[3] += f * double(hxy);
-        v[4] += f * double(hxz);
-        v[5] += f * double(hyz);
-      }
-    }
+    float h[6];
+    local_terms<Q, kKind>(pw + tid, TPB, s_L, 0, 1, h);
+    add_far<kKind>(h, inv_s, a, i, v);
     if (act) Body::epilogue(a, sc, i, td, v);
   }
   if (failed && tid == 0) {
@@ -889,6 +898,180 @@ __global__ void __launch_bounds__(TPB) k_fmm_p2p(const P2PArgs p, const AllPairs
       if (!mbar_wait_bounded(&bar[uu % kP2PStages], (uu / kP2PStages) & 1u)) drained = false;
     }
     if (!drained) atomicExch(a.err, MF_DEVERR_DRAIN_TIMEOUT);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Near field + L2P + epilogue, four targets of a leaf box per warp and round.
+// The lanes split the box's near source items: every lane holds the same four
+// targets and reads its own item, straight from the pair-layout records (a
+// warp's loads are one contiguous run), the next one while the current one is
+// swept, so a box of any count leaves at most three slots of its last round
+// empty and no wait is longer than a warp's own.  The CTA of 128 targets
+// (k_fmm_p2p) leaves 38 % of its lanes idle at 20 particles a box and waits for
+// its staging at four warps' pace.
+// Bound: the FP32 FMA pipe with the record loads behind it: 8 bytes from L1
+// or L2 per pair, which is why big boxes in great number stay with the staged
+// kernel (launch_near).  128 registers, 16 warps per SM.
+// Whole step of 200,003 particles (boxes of ~20) 13.69 -> 11.57 ms, of 330,000
+// (few boxes of ~155) 29.86 -> 23.78, field product of 150,000 sources at
+// 30,011 separate targets 1.97 -> 1.32 ms, tensor 3.89 -> 2.68.  Other splits of the
+// 32 lanes (targets per lane x lane groups), the same step at 200,003: 4 x 16
+// 12.31, 4 x 8 12.58, 2 x 16 11.99, 8 x 32 12.69, 2 x 4 14.33 ms.
+// ---------------------------------------------------------------------------
+constexpr int kNearT = 4;         // targets of a round
+constexpr int kNearFold = 64;     // items of a lane between folds of its FP32 sums
+constexpr int kNearMaxWarps = 8;  // warps per CTA (one box), taking rounds in turn
+template <int Q>
+struct NearWarp {
+  static constexpr int kHead = (ncoef(Q) - 1 + 3) & ~3;       // words per CTA: the box's locals
+  static constexpr int kWords = 64 + 3 * Q * kNearT;          // and per warp: rows, powers
+  static constexpr int smem(int warps) { return (kHead + warps * kWords) * int(sizeof(float)); }
+};
+
+template <int Q, int kKind>
+__global__ void __launch_bounds__(32 * kNearMaxWarps, 2)
+    k_fmm_near_warp(const P2PArgs p, const AllPairsArgs<float> a, const SceneDesc<float> sc) {
+  using Body = std::conditional_t<kKind == 0, FieldF2Body, std::conditional_t<kKind == 1, ForceF2Body, TensorF2Body>>;
+  using Item = PairItems::Item;
+  constexpr int kOut = Body::kOut;
+  using S = NearWarp<Q>;
+  static_assert(S::kHead % 2 == 0 && S::kWords % 2 == 0, "the rows are read as int2");
+  extern __shared__ __align__(16) float near_smem[];
+  if (p.done && *p.done != 0.0) return;
+  const FmmLevel& lv = p.lv;
+  const int64_t c = blockIdx.x;
+  const int32_t n = p.tcnt[c];
+  if (n == 0) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int ix = int(c % lv.nx), iy = int((c / lv.nx) % lv.ny), iz = int(c / (int64_t(lv.nx) * lv.ny));
+  const int32_t st0 = p.tstart[c];
+  float* s_L = near_smem;
+  float* ws = near_smem + S::kHead + warp * S::kWords;
+  int2* s_row = reinterpret_cast<int2*>(ws);  // per row: end in the flat item order, item offset
+  float* pw = ws + 64;                        // [3 Q][kNearT]
+  for (int k = threadIdx.x; k < ncoef(Q) - 1; k += blockDim.x) s_L[k] = p.L[int64_t(k) * lv.nbox + c];
+  __syncthreads();  // the only block barrier: the warps part ways here
+  for (int t0 = warp * kNearT; t0 < n; t0 += nw * kNearT) {
+    typename Body::TData td[kNearT];
+    float run[kNearT][kOut], cmp[kNearT][kOut];
+#pragma unroll
+    for (int t = 0; t < kNearT; ++t) {
+      Body::load(a, p.tperm[st0 + (t0 + t < n ? t0 + t : 0)], td[t]);
+#pragma unroll
+      for (int q = 0; q < kOut; ++q) run[t][q] = cmp[t][q] = 0.f;
+    }
+    for (int r0 = 0; r0 < p.n_rows; r0 += 32) {
+      // One lane per row of near boxes: its first item and its item count.
+      int b = 0, m = 0;
+      if (r0 + lane < p.n_rows) {
+        const int4 rw = p.rows[r0 + lane];
+        const int cy = iy + rw.y, cz = iz + rw.z;
+        if (cy >= 0 && cy < lv.ny && cz >= 0 && cz < lv.nz) {
+          const int cx0 = max(ix - rw.x, 0), cx1 = min(ix + rw.x, lv.nx - 1);
+          const int64_t rb = (int64_t(cz) * lv.ny + cy) * lv.nx;
+          b = p.start[rb + cx0] >> 1;
+          m = (p.start[rb + cx1 + 1] >> 1) - b;
+        }
+      }
+      int end = m;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, end, d);
+        if (lane >= d) end += up;
+      }
+      const int total = __shfl_sync(0xffffffffu, end, 31);
+      __syncwarp();  // the rows before these are done with
+      s_row[lane] = make_int2(end, b - (end - m));
+      __syncwarp();
+      int row = -1, row_end = 0, row_off = 0;
+      // Past the last item: a zero dipole, which adds nothing.
+      auto fetch = [&](int j) {
+        if (j >= total) return Item{{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+        while (j >= row_end) {  // ends at the last row: j < total, its end
+          const int2 e = s_row[++row];
+          row_end = e.x;
+          row_off = e.y;
+        }
+        return Body::load_item(p.pos2s, p.mom2s, j + row_off);
+      };
+      Item it = fetch(lane);
+      for (int j0 = 0; j0 < total; j0 += 32 * kNearFold) {
+        typename Body::Acc acc[kNearT];
+#pragma unroll
+        for (int t = 0; t < kNearT; ++t) acc[t].zero();
+        const int j1 = min(total, j0 + 32 * kNearFold);
+        for (int j = j0; j < j1; j += 32) {
+          const Item nx = fetch(j + 32 + lane);
+#pragma unroll
+          for (int t = 0; t < kNearT; ++t) Body::pair(td[t], it, sc.pc, acc[t]);
+          it = nx;
+        }
+#pragma unroll
+        for (int t = 0; t < kNearT; ++t) {
+          float o[kOut];
+          Body::tile_out(acc[t], o);
+#pragma unroll
+          for (int q = 0; q < kOut; ++q) comp_add(run[t][q], cmp[t][q], o[q]);
+        }
+      }
+    }
+    // The lanes' sums, in a fixed order: the first two exchanges leave a lane
+    // with target lane / 8, the others add up its eight lanes.
+    auto fold = [&](float& r, float& e, float sr, float se, int d) {
+      const float o = __shfl_xor_sync(0xffffffffu, sr, d), oe = __shfl_xor_sync(0xffffffffu, se, d);
+      comp_add(r, e, o);
+      e += oe;
+    };
+    auto scatter = [&](int keep, int d) {  // targets [0, 2 keep) -> [0, keep)
+      const bool hi = lane & d;
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (t >= keep) break;
+#pragma unroll
+        for (int q = 0; q < kOut; ++q) {
+          const float sr = hi ? run[t][q] : run[t + keep][q], se = hi ? cmp[t][q] : cmp[t + keep][q];
+          run[t][q] = hi ? run[t + keep][q] : run[t][q];
+          cmp[t][q] = hi ? cmp[t + keep][q] : cmp[t][q];
+          fold(run[t][q], cmp[t][q], sr, se, d);
+        }
+      }
+    };
+    scatter(2, 16);
+    scatter(1, 8);
+#pragma unroll
+    for (int q = 0; q < kOut; ++q)
+#pragma unroll
+      for (int d = 4; d > 0; d >>= 1) fold(run[0][q], cmp[0][q], run[0][q], cmp[0][q], d);
+    // Far field from the box's local expansion: eight lanes per target, each
+    // every eighth term.
+    const int tt = lane >> 3, tg = lane & 7;
+    const bool act = t0 + tt < n;
+    const int32_t i = p.tperm[st0 + (act ? t0 + tt : 0)];
+    const float inv_s = 1.f / lv.side;
+    if (tg < 3) {
+      const float4 tp = a.tpos[i];
+      const float x = tg == 0 ? tp.x : tg == 1 ? tp.y : tp.z, o = tg == 0 ? lv.ox : tg == 1 ? lv.oy : lv.oz;
+      const int ib = tg == 0 ? ix : tg == 1 ? iy : iz;
+      power_table<Q>((x - (o + (float(ib) + 0.5f) * lv.side)) * inv_s, pw + tg * Q * kNearT + tt, kNearT);
+    }
+    __syncwarp();
+    float h[6];
+    local_terms<Q, kKind>(pw + tt, kNearT, s_L, tg, 8, h);
+#pragma unroll
+    for (int q = 0; q < (kKind == 0 ? 3 : 6); ++q)
+#pragma unroll
+      for (int d = 4; d > 0; d >>= 1) h[q] += __shfl_xor_sync(0xffffffffu, h[q], d);
+    if (tg == 0 && act) {
+      double v[kOut];
+#pragma unroll
+      for (int q = 0; q < kOut; ++q) v[q] = double(run[0][q]) + double(cmp[0][q]);
+      add_far<kKind>(h, inv_s, a, i, v);
+      typename Body::TData t1;
+      Body::load(a, i, t1);
+      Body::epilogue(a, sc, i, t1, v);
+    }
+    __syncwarp();  // the powers are read before the next round writes them
   }
 }
 
@@ -1522,14 +1705,26 @@ mf_status Fmm::product(int kind, const float4* pos4, const float4* smom, const A
 }
 
 namespace {
-// One CTA of 128 threads per leaf box, 256-source stages, also for small
-// boxes: 64 threads with 128-source stages measured slower at 262,144
-// particles (boxes of <= 40: near field 3.9 against 2.7 ms for the field,
-// 11.3 against 7.3 for the force): the step and barrier count per box doubles.
-template <int Q, int kKind, bool kParts>
-void launch_p2p(unsigned grid, cudaStream_t st, const P2PArgs& pp, const AllPairsArgs<float>& a,
-                const SceneDesc<float>& sc) {
-  k_fmm_p2p<Q, kKind, kParts, 128, 256><<<grid, 128, p2p_smem<256>(), st>>>(pp, a, sc);
+// The near field of a product: four targets per warp (k_fmm_near_warp), as many
+// warps per box as a mean box has rounds, up to eight (steps at 200,003
+// particles, boxes of 16 on average: 2-4 warps 11.6-11.7 ms, 8 12.1; at
+// 330,000, few boxes of 81: 2 warps 28.6, 8 23.8).  The staged CTA of 128 targets
+// per box (k_fmm_p2p) is kept for the field where there are many boxes whose
+// targets nearly fill it: at 1,048,576 particles (12,800 boxes of 82 on
+// average) the step takes 54.4 ms with it against 55.7, while at 800,000 (62) it
+// takes 43.3 against 41.2 and in 4,074 boxes of 81 29.9 against 23.8.
+template <int Q, int kKind>
+void launch_near(unsigned boxes, int64_t nt, cudaStream_t st, const P2PArgs& pp, const AllPairsArgs<float>& a,
+                 const SceneDesc<float>& sc) {
+  if constexpr (kKind == 0) {
+    if (boxes >= 8192 && nt > 64 * int64_t(boxes) && nt <= 128 * int64_t(boxes)) {
+      k_fmm_p2p<Q, 0, false, 128, 256><<<boxes, 128, p2p_smem<256>(), st>>>(pp, a, sc);
+      return;
+    }
+  }
+  const int64_t rounds = (nt + int64_t(boxes) * kNearT - 1) / (int64_t(boxes) * kNearT);
+  const int warps = int(std::min<int64_t>(kNearMaxWarps, std::max<int64_t>(1, rounds)));
+  k_fmm_near_warp<Q, kKind><<<boxes, 32 * warps, NearWarp<Q>::smem(warps), st>>>(pp, a, sc);
 }
 }  // namespace
 
@@ -1642,13 +1837,13 @@ mf_status Fmm::product_q(int kind, const float4* pos4, const float4* smom, const
     ns.done = done;
     k_fmm_near_sym<<<unsigned((leaf.nbox + kNearSymWarps - 1) / kNearSymWarps), 32 * kNearSymWarps, 0, st>>>(ns, a, sc);
     ++nl;
-    launch_p2p<Q, 1, true>(unsigned(leaf.nbox), st, pp, a, sc);
+    k_fmm_p2p<Q, 1, true, 128, 256><<<unsigned(leaf.nbox), 128, p2p_smem<256>(), st>>>(pp, a, sc);
   } else if (kind == 1)
-    launch_p2p<Q, 1, false>(unsigned(leaf.nbox), st, pp, a, sc);
+    launch_near<Q, 1>(unsigned(leaf.nbox), nt_, st, pp, a, sc);
   else if (kind == 2)
-    launch_p2p<Q, 2, false>(unsigned(leaf.nbox), st, pp, a, sc);
+    launch_near<Q, 2>(unsigned(leaf.nbox), nt_, st, pp, a, sc);
   else
-    if constexpr (Q <= kMaxFieldDegree) launch_p2p<Q, 0, false>(unsigned(leaf.nbox), st, pp, a, sc);
+    if constexpr (Q <= kMaxFieldDegree) launch_near<Q, 0>(unsigned(leaf.nbox), nt_, st, pp, a, sc);
   ++nl;
   if (marks) MF_CUDA_TRY(cudaEventRecord(marks[3], st));
   launches_ = nl;
