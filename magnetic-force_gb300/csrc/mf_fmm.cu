@@ -7,7 +7,7 @@
 // whole product stays on the device:
 //   * one uniform box grid per level (level 0 is one box around the scene);
 //     the leaf level is the deepest with >= leaf_min particles per box on
-//     average, so a leaf box fills a 128-thread block of the near-field kernel;
+//     average (default 12), deep enough that few pairs of a near box are far apart;
 //   * particles binned into leaf boxes in row-major order (x fastest), each
 //     box's list in increasing particle index and padded to an even length,
 //     so every run of x-adjacent boxes is one contiguous, pair-aligned range of
@@ -722,18 +722,16 @@ __device__ __forceinline__ void add_far(const float* h, float inv_s, const AllPa
   }
 }
 
-// kKind: 0 field (H), 1 Kelvin force (contracted with the target dipole),
-// 2 force tensor (the Hessian kernel's 3x3 at each target).
-// kParts (force, targets = sources): the near field is not swept here but
-// added from k_fmm_near_sym's partial sums -- the box's own plane, then the
-// plane of every writer box (this box minus a half-stencil offset, inside the
-// grid and not empty), in a fixed order with compensated FP32.
+// kKind: 0 field (H); 1 Kelvin force, with kParts (targets = sources): the near
+// field is not swept here but added from k_fmm_near_sym's partial sums -- the
+// box's own plane, then the plane of every writer box (this box minus a
+// half-stencil offset, inside the grid and not empty), in a fixed order with
+// compensated FP32.
 template <int Q, int kKind, bool kParts, int TPB, int TILE>
 __global__ void __launch_bounds__(TPB) k_fmm_p2p(const P2PArgs p, const AllPairsArgs<float> a,
                                                          const SceneDesc<float> sc) {
-  static_assert(!kParts || kKind == 1, "partial sums: the Kelvin force only");
-  using Body = std::conditional_t<kKind == 0, FieldF2Body, std::conditional_t<kKind == 1, ForceF2Body, TensorF2Body>>;
-  constexpr bool kForce = kKind == 1;
+  static_assert(kKind == (kParts ? 1 : 0), "the field swept, or the Kelvin force from partial sums");
+  using Body = std::conditional_t<kKind == 0, FieldF2Body, ForceF2Body>;
   constexpr int kOut = Body::kOut;
   constexpr int NC = ncoef(Q) - 1;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -915,9 +913,11 @@ __global__ void __launch_bounds__(TPB) k_fmm_p2p(const P2PArgs p, const AllPairs
 // empty and no wait is longer than a warp's own.  The CTA of 128 targets
 // (k_fmm_p2p) leaves 38 % of its lanes idle at 20 particles a box and waits for
 // its staging at four warps' pace.
-// Bound: the FP32 FMA pipe with the record loads behind it: 8 bytes from L1
-// or L2 per pair, which is why big boxes in great number stay with the staged
-// kernel (launch_near).  128 registers, 16 warps per SM.
+// Bound: the packed FMAs' latency and register ports at three warps per
+// scheduler (128 registers; FMA pipe 50 %, issue 52 % at 200,003 particles), with
+// the record loads behind them: 8 bytes from L1 or L2 per pair (LSU wavefronts
+// 49 %), which is why big boxes in great number stay with the staged kernel
+// (launch_near).  Unrolling the item loop loses 8 % at 330,000 particles.
 // Whole step of 200,003 particles (boxes of ~20) 13.69 -> 11.57 ms, of 330,000
 // (few boxes of ~155) 29.86 -> 23.78, field product of 150,000 sources at
 // 30,011 separate targets 1.97 -> 1.32 ms, tensor 3.89 -> 2.68.  Other splits of the
