@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(128) k_correction_at(const CellGrid* __restric
         const float ds = dx * mj.x + dy * mj.y + dz * mj.z;
         if (kTensor) {
           float P, Q;
-          force_near_pq(r2, s_tbl, g.pc.inv_h, g.pc.ih4_over_k, P, Q);
+          force_near_pq_rn(r2, s_tbl, g.pc.inv_h, g.pc.ih4_over_k, P, Q);
           const float dP = P - cA, dQ = Q - cB;
           const float pd = dP * ds, qd = dQ * ds;
           const float ax = dP * mj.x, ay = dP * mj.y, az = dP * mj.z;

@@ -445,14 +445,36 @@ __device__ __forceinline__ void force_pair_sel(float dx, float dy, float dz, flo
   f[2] += dz * w + mz * u + sz * v;
 }
 
-// (P, Q) of the force tensor for any pair, FP32 without a branch (k.tbl set).
-__device__ __forceinline__ void force_coeffs_sel(float r2, const PairConsts<float>& k, float& P, float& Q) {
-  float Pn, Qn;
-  force_near_pq(r2, k.tbl, k.inv_h, k.ih4_over_k, Pn, Qn);
-  const float ri = rsqrt_approx(r2), ri2 = ri * ri, ri5 = ri2 * ri2 * ri;
-  const bool far = r2 > k.near2_force, apart = r2 > 0.f;
-  P = far ? ri5 : apart ? Pn : 0.f;
-  Q = far ? -5.f * ri5 * ri2 : apart ? Qn : 0.f;
+// (P, Q) of the force tensor for 0 < r <= 4h, in units of K, with r and 1/r to
+// FP32 rounding (one Newton step each from the hardware's reciprocal root):
+// the curves jump where their pieces meet, and a distance exactly on a join
+// has to stay on its side, as with a rounded square root (a root that is a
+// unit off puts the tensor at q = 3 1.3e-5 from its value, 4e-6 with this).
+__device__ __forceinline__ void force_near_pq_rn(float r2, const float* __restrict__ tbl, float inv_h,
+                                                 float ih4_over_k, float& P, float& Q) {
+  const float y = rsqrt_approx(r2);
+  float r = r2 * y;
+  r = fmaf(fmaf(-r, r, r2), 0.5f * y, r);
+  const float ri = fmaf(y, fmaf(-r, y, 1.f), y);
+  float c1, c2;
+  force_curves(r * inv_h, tbl, c1, c2);
+  const float s = ih4_over_k * ri;
+  P = c1 * s;
+  Q = fmaf(-3.f, c1, c2) * s * (ri * ri);
+}
+
+// (P, Q) of the force tensor for any pair, FP32 (k.tbl set).  A branch, not a
+// select: the external dipoles and the probe points this serves are mostly
+// farther than 4h from every source, and a warp whose lanes all are skips the
+// curves.
+__device__ __forceinline__ void force_coeffs_near_far(float r2, const PairConsts<float>& k, float& P, float& Q) {
+  const float ri = rsqrt_approx(r2), ri2 = ri * ri;
+  P = ri2 * ri2 * ri;
+  Q = -5.f * P * ri2;
+  if (r2 <= k.near2_force) {
+    P = Q = 0.f;
+    if (r2 > 0.f) force_near_pq_rn(r2, k.tbl, k.inv_h, k.ih4_over_k, P, Q);
+  }
 }
 
 // One tensor pair (6 unique entries xx, yy, zz, xy, xz, yz): t += T(d, s) / K.
@@ -461,7 +483,7 @@ __device__ __forceinline__ void tensor_pair(Real dx, Real dy, Real dz, Real sx, 
                                             const PairConsts<Real>& k, Real* t) {
   Real r2 = dx * dx + dy * dy + dz * dz;
   Real P, Q;
-  if constexpr (sizeof(Real) == 4) force_coeffs_sel(r2, k, P, Q);
+  if constexpr (sizeof(Real) == 4) force_coeffs_near_far(r2, k, P, Q);
   else force_coeffs(r2, k, P, Q);
   Real ds = dx * sx + dy * sy + dz * sz;
   Real pd = P * ds, qd = Q * ds;
