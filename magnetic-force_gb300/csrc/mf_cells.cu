@@ -256,6 +256,7 @@ __global__ void k_gather_sorted(const int32_t* __restrict__ perm, const float4* 
 // itself, for the force) get zero coefficients.
 struct NearConsts {
   float near2, h, inv_h, ih3_30, ih5_30, ih4k, cA, cB;
+  float c3;  // 3 ih5_unit: the field's alphas (ih5_30, cA) are in units of ih5_unit
 };
 struct NearTargets {  // two targets: positions, then dipoles (force)
   float4 xy, zm, mm;  // (x0, x1, y0, y1), (z0, z1, mx0, mx1), (my0, my1, mz0, mz1)
@@ -295,9 +296,9 @@ __device__ __forceinline__ void near_pair2(const NearTargets& t, const NearSourc
     float2 al, be;
     field_near_unit2(r2, c.h, c.inv_h, al, be);
     float2 da = f2_fma(al, f2_dup(c.ih5_30), f2_dup(-c.cA)), db = f2_fma(be, f2_dup(-c.ih3_30), f2_dup(c.cB));
-    da = make_float2(in0 ? da.x : 0.f, in1 ? da.y : 0.f);
+    da = make_float2(in0 && r2.x > 0.f ? da.x : 0.f, in1 && r2.y > 0.f ? da.y : 0.f);
     db = make_float2(in0 ? db.x : 0.f, in1 ? db.y : 0.f);
-    const float2 t3 = f2_mul(f2_mul(ds, f2_dup(3.f)), da);
+    const float2 t3 = f2_mul(f2_mul(ds, da), f2_dup(c.c3));
     acc[0] = f2_fma(dx, t3, f2_fma(s.mx, db, acc[0]));
     acc[1] = f2_fma(dy, t3, f2_fma(s.my, db, acc[1]));
     acc[2] = f2_fma(dz, t3, f2_fma(s.mz, db, acc[2]));
@@ -362,10 +363,12 @@ __global__ void __launch_bounds__(128) k_correction_cells(const CellGrid* __rest
     nc.h = g.pc.h;
     nc.inv_h = g.pc.inv_h;
     nc.ih3_30 = g.pc.ih3_30;
-    nc.ih5_30 = g.pc.ih5_30;
+    nc.ih5_30 = g.ih5_30;
     nc.ih4k = g.pc.ih4_over_k;
     if (kForce) clamped_force_coeffs(nc.near2, nc.cA, nc.cB);
     else clamped_field_coeffs(nc.near2, nc.cA, nc.cB);
+    nc.c3 = 3.f * g.ih5_unit;
+    if (!kForce) nc.cA *= 1.f / g.ih5_unit;
     const float cs = 1.f / g.inv_cs;
     // Row list of this cell: slot i = (dy, dz) in row-major order; a row
     // outside the grid or beyond the near radius has length 0.
@@ -498,6 +501,8 @@ __global__ void __launch_bounds__(128) k_correction_at(const CellGrid* __restric
   float cA, cB;
   if (kTensor) clamped_force_coeffs(near2, cA, cB);
   else clamped_field_coeffs(near2, cA, cB);
+  const float c3 = 3.f * g.ih5_unit;  // the field's alphas are in units of ih5_unit
+  if (!kTensor) cA *= 1.f / g.ih5_unit;
   const int side = 2 * R + 1, n_slots = side * side;
   const int64_t n_warps = int64_t(gridDim.x) * (blockDim.x >> 5);
   for (int64_t i = int64_t(blockIdx.x) * (blockDim.x >> 5) + wi; i < nt; i += n_warps) {
@@ -576,7 +581,7 @@ __global__ void __launch_bounds__(128) k_correction_at(const CellGrid* __restric
         } else {
           float al, be;
           field_near_unit(r2, near_rsqrt(r2), g.pc.h, g.pc.inv_h, al, be);
-          const float t3 = 3.f * ds * fmaf(al, g.pc.ih5_30, -cA);
+          const float t3 = r2 > 0.f ? c3 * (ds * fmaf(al, g.ih5_30, -cA)) : 0.f;
           const float db = fmaf(be, g.pc.ih3_30, -cB);
           acc[0] += dx * t3 - mj.x * db;
           acc[1] += dy * t3 - mj.y * db;
@@ -689,6 +694,9 @@ mf_status CellList::build(const float4* pos4, const std::vector<CellSceneSpec>& 
     g.n = scenes[s].n;
     g.k_off = prefix;
     g.pc = make_pair_consts<float>(h);
+    const double ih5 = 1.0 / (30.0 * h * h * h * h * h);
+    g.ih5_unit = ih5 < 0x1p-100 ? 0x1p-96f : 1.f;
+    g.ih5_30 = float(std::min(ih5 / double(g.ih5_unit), 3.4e38));
     cells += int64_t(g.nx) * g.ny * g.nz;
     prefix += scenes[s].n;
   }

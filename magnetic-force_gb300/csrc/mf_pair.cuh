@@ -54,7 +54,13 @@ __host__ __device__ inline PairConsts<Real> make_pair_consts(double h) {
   k.h = Real(h);
   k.ih3 = Real(1.0 / (h * h * h));
   k.ih3_30 = Real(1.0 / (30.0 * h * h * h));
-  k.ih5_30 = Real(1.0 / (30.0 * h * h * h * h * h));
+  // h^-5 leaves FP32 from 1e-8 down, where it is held finite: what it scales
+  // overflows there, except at r = 0, which the kernels leave out.  Above 1e7
+  // it is subnormal: the corrections take theirs times a power of two
+  // (CellGrid); here the multiplication that would undo it costs 1.5 % of every
+  // small solve (field of 200 particles at h = 4e7: 9e-7 from FP64).
+  const double ih5 = 1.0 / (30.0 * h * h * h * h * h);
+  k.ih5_30 = Real(sizeof(Real) == 4 ? fmin(ih5, 3.4e38) : ih5);
   k.ih4_over_k = Real(1.0 / (h * h * h * h * kForceK));
   k.near2_field = Real(4.0 * h * h);
   k.near2_force = Real(16.0 * h * h);
@@ -312,7 +318,8 @@ __device__ __forceinline__ void clamped_force_coeffs(float near2, float& P, floa
 // Field: 30 alpha h^5 and 30 beta h^3 at q = r / h < 2.  Times 30 every
 // coefficient is a whole number: 0.8f alone would put 4e-7 of alpha at q = 2
 // into every pair.  The outer piece's beta is written in t = 2 - q, where its
-// terms do not cancel.
+// terms do not cancel.  alpha is infinite at r = 0 from h = 2e-8 down; it
+// multiplies d = 0 there and is to be taken as 0.
 //   q < 1: 24 - 15 q,                       -80 + 144 q^2 - 75 q^3
 //   else:  5 q - 24 + 30 / q - 2 q^-5,      4 + 6 t + 6 t^2 - 25 t^3 - 2 q^-3
 // ri: near_rsqrt(r2), finite at r = 0 (where q comes out 0).
@@ -416,6 +423,7 @@ __device__ __forceinline__ void field_pair_sel(float dx, float dy, float dz, flo
   float al, be;
   field_near_unit(r2, ri, k.h, k.inv_h, al, be);
   const bool far = r2 >= k.near2_field;
+  al = r2 > 0.f ? al : 0.f;
   const float beta = far ? ri3 : be * k.ih3_30;
   const float alpha = far ? ri3 * ri2 : al * k.ih5_30;
   const float t = (dx * sx + dy * sy + dz * sz) * alpha;
