@@ -146,6 +146,7 @@ mf_status Scratch::check(cudaStream_t st) {
     MF_CUDA_TRY(cudaMemsetAsync(err.ptr, 0, err.bytes, st));
     if (counters.ptr) MF_CUDA_TRY(cudaMemsetAsync(counters.ptr, 0, counters.bytes, st));
     MF_CUDA_TRY(cudaStreamSynchronize(st));
+    if (host == MF_DEVERR_NONFINITE) return fail(MF_ERR_INVALID_ARG, "non-finite positions");
     char buf[128];
     snprintf(buf, sizeof(buf), "kernel wait ran out (device error %d); results of that launch are invalid",
              int(host));

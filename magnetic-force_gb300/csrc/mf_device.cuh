@@ -15,6 +15,7 @@ enum : int {
   MF_DEVERR_NONE = 0,
   MF_DEVERR_STAGE_TIMEOUT = 1,   // a source tile never arrived in shared memory
   MF_DEVERR_DRAIN_TIMEOUT = 2,   // copies still in flight when leaving after an error
+  MF_DEVERR_NONFINITE = 3,       // a direct call's source positions are not finite
 };
 
 // Try-wait iterations before a staging wait gives up.  Each try_wait blocks

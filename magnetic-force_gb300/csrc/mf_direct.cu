@@ -15,13 +15,36 @@
 namespace mfgb {
 namespace {
 
-__global__ void k_pack_aos(int64_t n, const float* __restrict__ src, float4* __restrict__ dst) {
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    dst[i] = make_float4(src[3 * i], src[3 * i + 1], src[3 * i + 2], 0.f);
+// AoS [n][3] -> records.  reset (optional) is cleared; seen (optional) gets bit
+// k if a value of axis k is not NaN and bit 3 if any value is infinite.
+__global__ void k_pack_aos(int64_t n, const float* __restrict__ src, float4* __restrict__ dst,
+                           int32_t* __restrict__ reset = nullptr, int32_t* __restrict__ seen = nullptr) {
+  if (reset && blockIdx.x == 0 && threadIdx.x == 0) *reset = 0;
+  int32_t f = 0;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+    const float x = src[3 * i], y = src[3 * i + 1], z = src[3 * i + 2];
+    dst[i] = make_float4(x, y, z, 0.f);
+    f |= (isnan(x) ? 0 : 1) | (isnan(y) ? 0 : 2) | (isnan(z) ? 0 : 4) | (isinf(x) || isinf(y) || isinf(z) ? 8 : 0);
+  }
+  if (seen) {
+    __shared__ int32_t s_f;
+    if (threadIdx.x == 0) s_f = 0;
+    __syncthreads();
+    f = __reduce_or_sync(0xffffffffu, f);
+    if ((threadIdx.x & 31) == 0 && f) atomicOr(&s_f, f);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_f) atomicOr(seen, s_f);
+  }
 }
 
-// SoA (k arrays of n) -> AoS [n][k]
-__global__ void k_soa_to_aos_k(int64_t n, int k, const float* __restrict__ soa, float* __restrict__ aos) {
+// SoA (k arrays of n) -> AoS [n][k].  seen (optional, k_pack_aos over the
+// sources): without a finite bounding box nothing is written and err is set.
+__global__ void k_soa_to_aos_k(int64_t n, int k, const float* __restrict__ soa, float* __restrict__ aos,
+                               const int32_t* __restrict__ seen = nullptr, int32_t* __restrict__ err = nullptr) {
+  if (seen && *seen != 7) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(err, 0, MF_DEVERR_NONFINITE);
+    return;
+  }
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     for (int c = 0; c < k; ++c) aos[i * k + c] = soa[int64_t(c) * n + i];
 }
@@ -51,7 +74,7 @@ constexpr double kPackedDirectMin = 1.25e8;
 
 struct DirectCtx {
   std::mutex mu;
-  DevBuf t4, s4, m4, tm4, soa, aux, s2, m2, corr;
+  DevBuf t4, s4, m4, tm4, soa, aux, s2, m2, corr, seen;
   Scratch scr;
   CellList cells;
   Plan<float> plan[kBodies];
@@ -59,7 +82,7 @@ struct DirectCtx {
   int64_t plan_nt[kBodies] = {}, plan_ns[kBodies] = {};
   double plan_h[kBodies] = {};
   void release() {
-    for (DevBuf* b : {&t4, &s4, &m4, &tm4, &soa, &aux, &s2, &m2, &corr}) b->release();
+    for (DevBuf* b : {&t4, &s4, &m4, &tm4, &soa, &aux, &s2, &m2, &corr, &seen}) b->release();
     scr.partials.release();
     scr.counters.release();
     scr.err.release();
@@ -118,8 +141,13 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
   MF_TRY(c.s4.reserve(size_t(ns) * sizeof(float4)));
   MF_TRY(c.m4.reserve(size_t(ns) * sizeof(float4)));
   MF_TRY(c.soa.reserve(size_t(nt) * kOut * sizeof(float)));
-  k_pack_aos<<<grid_for(nt), 256, 0, st>>>(nt, targets, c.t4.as<float4>());
-  k_pack_aos<<<grid_for(ns), 256, 0, st>>>(ns, sources, c.s4.as<float4>());
+  MF_TRY(c.seen.reserve(sizeof(int32_t)));
+  // The cell list of the packed path refuses sources without a finite bounding
+  // box; the field and the force refuse them on the exact path as well.
+  const bool large = double(nt) * double(ns) >= kPackedDirectMin;
+  int32_t* seen = !large && body != Body::Tensor ? c.seen.as<int32_t>() : nullptr;
+  k_pack_aos<<<grid_for(nt), 256, 0, st>>>(nt, targets, c.t4.as<float4>(), seen);
+  k_pack_aos<<<grid_for(ns), 256, 0, st>>>(ns, sources, c.s4.as<float4>(), nullptr, seen);
   k_pack_aos<<<grid_for(ns), 256, 0, st>>>(ns, charges, c.m4.as<float4>());
   MF_CUDA_TRY(cudaGetLastError());
   LaunchIO<float> io;
@@ -127,9 +155,20 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
   io.spos = c.s4.as<float4>();
   io.smom = c.m4.as<float4>();
   // Large calls go through the packed two-source kernels: sources in pair
-  // layout, a cell list over the sources, and the near-field correction.
+  // layout, a cell list over the sources, and the near-field correction.  The
+  // tensor, which the exact kernel takes at any positions, goes there where no
+  // cell list can be made (positions that are not finite, or too spread).
   Body launch_body = body;
-  if (double(nt) * double(ns) >= kPackedDirectMin) {
+  bool packed = large;
+  if (packed) {
+    const mf_status built = c.cells.build(c.s4.as<float4>(), {CellSceneSpec{0, ns, double(h)}}, st);
+    if (built != MF_OK) {
+      if (body != Body::Tensor) return built;
+      cudaGetLastError();
+      packed = false;
+    }
+  }
+  if (packed) {
     const size_t pair_bytes = size_t(ns + 1) * sizeof(float4);
     MF_TRY(c.s2.reserve(pair_bytes));
     MF_TRY(c.m2.reserve(pair_bytes));
@@ -137,7 +176,6 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
     to_pairs(c.s4.as<float4>(), c.s2.as<float4>(), ns, st);
     to_pairs(c.m4.as<float4>(), c.m2.as<float4>(), ns, st);
     MF_CUDA_TRY(cudaGetLastError());
-    MF_TRY(c.cells.build(c.s4.as<float4>(), {CellSceneSpec{0, ns, double(h)}}, st));
     if (body == Body::Field) {
       if (targets == sources && nt == ns)
         MF_TRY(c.cells.field_correction(c.s4.as<float4>(), c.m4.as<float4>(), c.corr.as<float4>(), st));
@@ -183,7 +221,7 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
     }
   }
   MF_TRY(run_plan<float>(*plan, io, c.scr, st));
-  k_soa_to_aos_k<<<grid_for(nt), 256, 0, st>>>(nt, kOut, soa, results);
+  k_soa_to_aos_k<<<grid_for(nt), 256, 0, st>>>(nt, kOut, soa, results, seen, c.scr.err.as<int32_t>());
   MF_CUDA_TRY(cudaGetLastError());
   MF_TRY(c.scr.check(st));  // synchronises the stream
   return MF_OK;
