@@ -675,7 +675,7 @@ mf_status CellList::build(const float4* pos4, const std::vector<CellSceneSpec>& 
     double cs = h * (1.0 + 1e-4);
     // Keep the grid at most ~8 cells per particle: widen cells for sparse scenes.
     const double cap = std::max(64.0, 8.0 * double(scenes[s].n));
-    for (int it = 0; it < 64; ++it) {
+    for (int it = 0; it < 512; ++it) {  // any FP32 extent over any FP32 h (1.25^512 = 1e49)
       const double c3 = (std::floor(ext[0] / cs) + 1) * (std::floor(ext[1] / cs) + 1) * (std::floor(ext[2] / cs) + 1);
       if (c3 <= cap) break;
       cs *= 1.25;

@@ -52,3 +52,17 @@ def test_what_is_taken(mf, cuda, n, kind, refused):
     # and the next call is as if nothing had been
     good = dev(cuda, bad_sources(n, "finite")[0])
     assert bool(cuda.isfinite(mf.direct_field(good, good, dm, 0.1)).all())
+
+
+def test_tensor_of_sources_too_spread_for_cells(mf, cuda, oracle):
+    """Two clusters 1e6 apart at h = 1e-3: a cell list would need 1e9 cells a side."""
+    rng = np.random.default_rng(3)
+    s = rng.random((12000, 3)).astype(np.float32)
+    s[::2] += np.float32(1e6)
+    m = rng.normal(size=s.shape).astype(np.float32)
+    h = float(np.float32(1e-3))
+    got = mf.direct_force_tensor(dev(cuda, s), dev(cuda, s), dev(cuda, m), h).cpu().numpy()
+    k = np.r_[0:40, 11960:12000]
+    sd = s.astype(np.float64)
+    want = oracle.tensor_sum(sd[k], sd, m.astype(np.float64), h).reshape(-1, 9)
+    assert np.linalg.norm(got[k] - want) / np.linalg.norm(want) < 1e-5
