@@ -64,13 +64,42 @@ unsigned grid_for(int64_t n) {
 
 constexpr int kBodies = 6;
 
-// Target-source pairs from which the packed kernels beat the exact-branch
-// ones.  They need a cell list (ten launches, a host round trip) and the
-// near-field correction: whole calls at 4,000 x 4,000, 10,000 x 10,000 and
-// 12,000 x 12,000 take 176 / 264 / 303 us packed and 100 / 237 / 313 exact
-// for the field, 227 / 401 / 464 and 124 / 374 / 460 for the tensor, 217 /
-// 375 / 421 and 126 / 341 / 470 for the force.
-constexpr double kPackedDirectMin = 1.25e8;
+// Whether a call's packed kernels beat the exact-branch ones.  They cost a cell
+// list over the sources (ten launches, a host round trip, then with the count)
+// and the near-field correction, a warp per target; they save about half of
+// every pair of the padded target blocks.  Whole calls, exact / packed us:
+//   field, 64 x 200,000 746 / 513, 1,000 x 40,000 295 / 352, 4,000 x 40,000
+//   474 / 327, 40,000 x 4,000 405 / 346, 200,000 x 1,000 399 / 562; of one set
+//   (the correction by cells) 8,500 219 / 234, 9,000 333 / 261.
+//   force of one set, 10,000 358 / 333-405, 11,500 494 / 386-473 (few to many
+//   near pairs).
+//   tensor, 256 x 1,000,000 898 / 1,208, 1,000 x 200,000 644 / 624, 1,000 x
+//   1,000,000 2,033 / 1,480, 2,000 x 40,000 433 / 442, 11,000 x 10,000 424 /
+//   418, 40,000 x 10,000 1,331 / 976, 1,000,000 x 1,000 3,119 / 5,115.
+bool packed_pays(Body body, bool one_set, int64_t nt, int64_t ns) {
+  const double t = double(nt), s = double(ns);
+  auto padded = [&](int64_t block) { return double((nt + block - 1) / block * block) * s; };
+  if (body == Body::Tensor) return padded(128) >= 9e7 + 360.0 * s + 2450.0 * t;
+  if (one_set) return t * s >= (body == Body::Field ? 7.6e7 : 1.25e8);
+  return padded(512) >= 7.5e7 + 1000.0 * t;
+}
+
+// Where many pairs are near, the correction costs more than the packed kernel
+// saves.  near_part: the part of the sources expected within `reach` of a
+// target (bbox: theirs), from which on the exact kernel is taken.  12,000 x
+// 12,000 in the unit cube at h = 0.05, 0.1, 0.2, 0.4, exact / packed us: field
+// (2h: 0.4, 3, 27, 52 %) 309 / 285, 310 / 289, 312 / 1,007, 313 / 5,976; force
+// (4h: 3, 27, 52, 52 %) 482 / 379, 484 / 462, 484 / 1,428, 484 / 8,136; tensor
+// 458 / 366, 534 / 521, 542 / 874, 534 / 1,084.
+constexpr double kDenseField = 0.06, kDenseForce = 0.3;
+double near_part(const double* bbox, double reach) {
+  double f = kPi / 6.0;
+  for (int k = 0; k < 3; ++k) f *= std::min(1.0, 2.0 * reach / std::max(bbox[3 + k] - bbox[k], 1e-300));
+  return f;
+}
+bool dense(Body body, const double* bbox, double h) {
+  return body == Body::Field ? near_part(bbox, 2.0 * h) > kDenseField : near_part(bbox, 4.0 * h) > kDenseForce;
+}
 
 struct DirectCtx {
   std::mutex mu;
@@ -144,7 +173,8 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
   MF_TRY(c.seen.reserve(sizeof(int32_t)));
   // The cell list of the packed path refuses sources without a finite bounding
   // box; the field and the force refuse them on the exact path as well.
-  const bool large = double(nt) * double(ns) >= kPackedDirectMin;
+  const bool one_set = body == Body::Force || (targets == sources && nt == ns);
+  const bool large = packed_pays(body, one_set, nt, ns);
   int32_t* seen = !large && body != Body::Tensor ? c.seen.as<int32_t>() : nullptr;
   k_pack_aos<<<grid_for(nt), 256, 0, st>>>(nt, targets, c.t4.as<float4>(), seen);
   k_pack_aos<<<grid_for(ns), 256, 0, st>>>(ns, sources, c.s4.as<float4>(), nullptr, seen);
@@ -155,9 +185,9 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
   io.spos = c.s4.as<float4>();
   io.smom = c.m4.as<float4>();
   // Large calls go through the packed two-source kernels: sources in pair
-  // layout, a cell list over the sources, and the near-field correction.  The
-  // tensor, which the exact kernel takes at any positions, goes there where no
-  // cell list can be made (positions that are not finite, or too spread).
+  // layout, a cell list over the sources, and the near-field correction.  Dense
+  // ones go to the exact kernel, and so does a tensor whose sources no cell list
+  // can be made of (positions that are not finite: that kernel takes any).
   Body launch_body = body;
   bool packed = large;
   if (packed) {
@@ -165,6 +195,8 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
     if (built != MF_OK) {
       if (body != Body::Tensor) return built;
       cudaGetLastError();
+      packed = false;
+    } else if (dense(body, c.cells.bbox(0), h)) {
       packed = false;
     }
   }
@@ -177,7 +209,7 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
     to_pairs(c.m4.as<float4>(), c.m2.as<float4>(), ns, st);
     MF_CUDA_TRY(cudaGetLastError());
     if (body == Body::Field) {
-      if (targets == sources && nt == ns)
+      if (one_set)
         MF_TRY(c.cells.field_correction(c.s4.as<float4>(), c.m4.as<float4>(), c.corr.as<float4>(), st));
       else
         MF_TRY(c.cells.field_correction_at(c.t4.as<float4>(), nt, c.s4.as<float4>(), c.m4.as<float4>(),
@@ -200,8 +232,7 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
   // particles from kSymDirectMin particles on (no tuning on this path: a
   // call can be seconds long), per MF_PAIR_SYMMETRIC.
   int shape = 0;
-  if ((launch_body == Body::FieldF2 || launch_body == Body::ForceF2) &&
-      (body == Body::Force || (targets == sources && nt == ns))) {
+  if ((launch_body == Body::FieldF2 || launch_body == Body::ForceF2) && one_set) {
     const int mode = default_sym_mode();
     if (mode == 2 || (mode == 1 && nt >= kSymDirectMin)) shape = kShapeSym;
   }
