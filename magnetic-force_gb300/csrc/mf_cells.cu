@@ -660,6 +660,7 @@ mf_status CellList::build(const float4* pos4, const std::vector<CellSceneSpec>& 
   host_bbox_.assign(6 * size_t(ns), 0.0);
   for (size_t k = 0; k < hb.size(); ++k) host_bbox_[k] = double(ord2f(hb[k]));
   int64_t cells = 0, prefix = 0;
+  double spanned = 0.0;
   for (int s = 0; s < ns; ++s) {
     CellGrid& g = host_grids_[size_t(s)];
     const double h = scenes[s].h;
@@ -698,9 +699,13 @@ mf_status CellList::build(const float4* pos4, const std::vector<CellSceneSpec>& 
     g.ih5_unit = ih5 < 0x1p-100 ? 0x1p-96f : 1.f;
     g.ih5_30 = float(std::min(ih5 / double(g.ih5_unit), 3.4e38));
     cells += int64_t(g.nx) * g.ny * g.nz;
+    double box = 1.0;  // the particles' own bounding box, in cells
+    for (int c = 0; c < 3; ++c) box *= std::max(1.0, (ext[c] - 2.0 * margin_h * h) / cs);
+    spanned += box;
     prefix += scenes[s].n;
   }
   n_cells_ = cells;
+  full_ = double(n_total_) >= 2.0 * spanned;
   MF_TRY(grids_.reserve(sizeof(CellGrid) * size_t(ns)));
   MF_CUDA_TRY(cudaMemcpyAsync(grids_.ptr, host_grids_.data(), sizeof(CellGrid) * size_t(ns), cudaMemcpyHostToDevice,
                               st));
@@ -739,13 +744,17 @@ mf_status CellList::rebin(const float4* pos4, cudaStream_t st) {
   return MF_OK;
 }
 
-// Warps per cell of the correction.  The force always takes 4: its cells are
-// long (116 sweeps of 32 candidates at h = 2 spacings), and one warp each left
-// a last wave a fifth of the kernel long at 65,536 particles (743 against 573
-// us; 273 against 143 at 16,411).  The field's cells are short (19 sweeps), so
-// 4 warps pay while there are fewer cells than the device runs warps (14
-// against 39 us at 3,001 particles, 25 against 48 at 12,289), and one warp
-// from there on (24 scenes in one list: 25 against 41 us).
+// Warps per cell of the correction.  The force takes 4 where cells are full:
+// they are long (116 sweeps of 32 candidates at h = 2 spacings), and one warp
+// each left a last wave a fifth of the kernel long at 65,536 particles (743
+// against 573 us; 273 against 143 at 16,411).  Below two particles per cell of
+// the bounding boxes (h under 1.3-1.6 spacings) a cell's row list costs more
+// than its sweeps, and one warp each is better: whole direct forces of 20,000
+// particles, 4 warps / 1, 772 / 697 us at h = 0.5 spacings, 711 / 695 at 1.3,
+// 710 / 735 at 1.6.  The field's cells are short (19 sweeps), so 4 warps pay
+// while there are fewer cells than the device runs warps (14 against 39 us at
+// 3,001 particles, 25 against 48 at 12,289), and one warp from there on (24
+// scenes in one list: 25 against 41 us).
 constexpr int64_t kSplitCells = 8192;
 static unsigned cell_grid(int64_t cells) {
   int64_t g = cells;
@@ -810,7 +819,8 @@ mf_status CellList::force_correction(const float4* pos4, const float4* mom4, flo
                                      float4* mom2) const {
   k_gather_sorted<<<grid_for(n_total_), 256, 0, st>>>(perm_.as<int32_t>(), pos4, mom4, n_total_, spos_.as<float4>(),
                                                       smom_.as<float4>(), nullptr, 0, mom2);
-  k_correction_cells<true, 4><<<cell_grid(n_cells_), 128, 0, st>>>(
+  auto* k = full_ ? k_correction_cells<true, 4> : k_correction_cells<true, 1>;
+  k<<<cell_grid(full_ ? n_cells_ : (n_cells_ + 3) / 4), 128, 0, st>>>(
       grids_.as<CellGrid>(), n_scenes_, n_cells_, perm_.as<int32_t>(), cell_start_.as<int32_t>(), spos_.as<float4>(),
       smom_.as<float4>(), corr, skip_force_on_ ? skip_force_.as<int32_t>() : nullptr, nullptr, 0, nullptr, 0);
   MF_CUDA_TRY(cudaGetLastError());

@@ -431,6 +431,7 @@ class CellList {
   std::vector<CellGrid> host_grids_;
   std::vector<double> host_bbox_;
   int64_t n_total_ = 0, n_cells_ = 0;
+  bool full_ = true;  // two particles and more per cell of the scenes' bounding boxes
   int32_t n_scenes_ = 0;
 };
 
