@@ -296,7 +296,7 @@ __device__ __forceinline__ void near_pair2(const NearTargets& t, const NearSourc
     float2 al, be;
     field_near_unit2(r2, c.h, c.inv_h, al, be);
     float2 da = f2_fma(al, f2_dup(c.ih5_30), f2_dup(-c.cA)), db = f2_fma(be, f2_dup(-c.ih3_30), f2_dup(c.cB));
-    da = make_float2(in0 && r2.x > 0.f ? da.x : 0.f, in1 && r2.y > 0.f ? da.y : 0.f);
+    da = make_float2(in0 ? da.x : 0.f, in1 ? da.y : 0.f);
     db = make_float2(in0 ? db.x : 0.f, in1 ? db.y : 0.f);
     const float2 t3 = f2_mul(f2_mul(ds, da), f2_dup(c.c3));
     acc[0] = f2_fma(dx, t3, f2_fma(s.mx, db, acc[0]));
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(128) k_correction_at(const CellGrid* __restric
         } else {
           float al, be;
           field_near_unit(r2, near_rsqrt(r2), g.pc.h, g.pc.inv_h, al, be);
-          const float t3 = r2 > 0.f ? c3 * (ds * fmaf(al, g.ih5_30, -cA)) : 0.f;
+          const float t3 = c3 * (ds * fmaf(al, g.ih5_30, -cA));
           const float db = fmaf(be, g.pc.ih3_30, -cB);
           acc[0] += dx * t3 - mj.x * db;
           acc[1] += dy * t3 - mj.y * db;
@@ -696,8 +696,8 @@ mf_status CellList::build(const float4* pos4, const std::vector<CellSceneSpec>& 
     g.k_off = prefix;
     g.pc = make_pair_consts<float>(h);
     const double ih5 = 1.0 / (30.0 * h * h * h * h * h);
-    g.ih5_unit = ih5 < 0x1p-100 ? 0x1p-96f : 1.f;
-    g.ih5_30 = float(std::min(ih5 / double(g.ih5_unit), 3.4e38));
+    g.ih5_unit = ih5 < 0x1p-100 ? 0x1p-96f : ih5 > 0x1p+100 ? 0x1p+20f : 1.f;
+    g.ih5_30 = float(std::min(ih5 / double(g.ih5_unit), 1e37));  // times alpha's 24 at r = 0 still finite
     cells += int64_t(g.nx) * g.ny * g.nz;
     double box = 1.0;  // the particles' own bounding box, in cells
     for (int c = 0; c < 3; ++c) box *= std::max(1.0, (ext[c] - 2.0 * margin_h * h) / cs);

@@ -367,7 +367,7 @@ struct CellGrid {
   int32_t nx, ny, nz;
   int32_t reach_field;       // cells to scan each way for r < 2h
   int32_t reach_force;       // cells to scan each way for r <= 4h
-  float ih5_30, ih5_unit;    // 1/(30 h^5) in units of ih5_unit, a power of two that keeps it normal
+  float ih5_30, ih5_unit;    // 1/(30 h^5) in units of ih5_unit, a power of two that keeps it in range
   int64_t cell_off;          // first cell of this scene in the global arrays
   int64_t p_off, n;          // particle range of the scene
   int64_t k_off;             // particles of the scenes before this one
