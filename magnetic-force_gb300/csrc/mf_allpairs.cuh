@@ -99,6 +99,8 @@ struct RecordItems {
   // and 2.2e-7 from FP64 where the packed body gives 1.5e-7 and 1.4e-7; now
   // 1.2e-7 both, 5 % slower at 11,000.
   static constexpr int kFold = sizeof(Real) == 4 ? 64 : 128;
+  static constexpr int kGroup = 1;  // items a body takes at once (group())
+  static constexpr int kSources = 1;  // per item
   struct Item {
     R4 p, m;
   };
@@ -266,6 +268,7 @@ struct TensorBody : RecordItems<Real> {
   using R4 = typename Vec4T<Real>::type;
   static constexpr int kAcc = 6;
   static constexpr int kOut = 6;
+  static constexpr int kGroup = sizeof(Real) == 4 ? 4 : 1;
   struct TData {
     Real x, y, z;
   };
@@ -281,6 +284,38 @@ struct TensorBody : RecordItems<Real> {
     const R4& sp = it.p;
     const R4& sm = it.m;
     tensor_pair<Real>(t.x - sp.x, t.y - sp.y, t.z - sp.z, sm.x, sm.y, sm.z, pc, acc.v);
+  }
+  // kGroup items.  A warp skips the curves of the items none of its lanes is
+  // near (external dipoles and probe points are mostly farther than 4h from
+  // every source), and of three or four it is near takes all four at once: a
+  // branch for every item leaves each pair's chain of operations exposed.
+  // Whole calls, a branch per item / none / this: 1,000 x 1,000 98 / 85 / 89 us,
+  // 10 x 4,000,000 1.3 / 2.1 / 1.5 ms; the tensor of 6,000 dipoles beside 12,289
+  // particles 163 / 221 / 182 us.
+  __device__ static void group(const TData& t, const typename RecordItems<Real>::Item* it, const PairConsts<Real>& pc,
+                               Acc& acc) {
+    bool near[kGroup];
+    int n_near = 0;
+#pragma unroll
+    for (int g = 0; g < kGroup; ++g) {
+      const Real dx = t.x - it[g].p.x, dy = t.y - it[g].p.y, dz = t.z - it[g].p.z;
+      near[g] = __any_sync(0xffffffffu, dx * dx + dy * dy + dz * dz <= pc.near2_force);
+      n_near += near[g] ? 1 : 0;
+    }
+    if (n_near > 2) {
+#pragma unroll
+      for (int g = 0; g < kGroup; ++g) pair(t, it[g], pc, acc);
+      return;
+    }
+#pragma unroll
+    for (int g = 0; g < kGroup; ++g) {
+      const Real dx = t.x - it[g].p.x, dy = t.y - it[g].p.y, dz = t.z - it[g].p.z;
+      const Real r2 = dx * dx + dy * dy + dz * dz;
+      const Real ri = rsqrt_r<Real>(r2), ri2 = ri * ri;
+      Real P = ri2 * ri2 * ri, Q = Real(-5) * ri2 * P;
+      if (near[g]) force_coeffs_sel(r2, pc, P, Q);
+      tensor_terms<Real>(dx, dy, dz, it[g].m.x, it[g].m.y, it[g].m.z, P, Q, acc.v);
+    }
   }
   __device__ static void tile_out(const Acc& acc, Real* o) {
     const Real c = Real(kForceK);
@@ -315,6 +350,7 @@ struct TensorBody : RecordItems<Real> {
 // ----------------------------------------------------------------------------
 struct PairItems {
   static constexpr int kFold = 128;  // items: a whole tile
+  static constexpr int kGroup = 1, kSources = 2;
   struct Item {
     float2 x, y, z, mx, my, mz;
   };
@@ -586,13 +622,23 @@ __global__ void __launch_bounds__(TPB) allpairs_kernel(const AllPairsArgs<Real> 
       const R4* __restrict__ sp = stage_pos(s);
       const R4* __restrict__ sm = stage_mom(s);
       const int n_items = Body::items(cnt);
-      for (int j0 = 0; j0 < n_items; j0 += Body::kFold) {
+      // Items [j0, j1) of the tile, summed in plain FP32, into the running sums.
+      auto sweep = [&](int j0, int j1) {
         typename Body::Acc acc[TPT];
 #pragma unroll
         for (int t = 0; t < TPT; ++t) acc[t].zero();
-        const int j1 = min(n_items, j0 + Body::kFold);
+        int j = j0;
+        if constexpr (Body::kGroup > 1) {
+          for (; j + Body::kGroup <= j1; j += Body::kGroup) {
+            typename Body::Item it[Body::kGroup];
+#pragma unroll
+            for (int g = 0; g < Body::kGroup; ++g) it[g] = Body::load_item(sp, sm, j + g);
+#pragma unroll
+            for (int t = 0; t < TPT; ++t) Body::group(td[t], it, pc, acc[t]);
+          }
+        }
 #pragma unroll 4
-        for (int j = j0; j < j1; ++j) {
+        for (; j < j1; ++j) {
           const typename Body::Item it = Body::load_item(sp, sm, j);
 #pragma unroll
           for (int t = 0; t < TPT; ++t) Body::pair(td[t], it, pc, acc[t]);
@@ -606,6 +652,19 @@ __global__ void __launch_bounds__(TPB) allpairs_kernel(const AllPairsArgs<Real> 
             if constexpr (kComp) comp_add(run[t][q], cmp[t][q], o[q]);
             else run[t][q] += o[q];
           }
+        }
+      };
+      if constexpr (Body::kFold * Body::kSources >= TILE) {
+        sweep(0, n_items);
+      } else {
+        // (whole tiles apart: with a run-time end the compiler kept the 256 x 2
+        // field body to 64 registers, and direct fields took 8 % longer)
+        if (n_items == TILE) {
+#pragma unroll 1
+          for (int j0 = 0; j0 < TILE; j0 += Body::kFold) sweep(j0, j0 + Body::kFold);
+        } else {
+#pragma unroll 1
+          for (int j0 = 0; j0 < n_items; j0 += Body::kFold) sweep(j0, min(n_items, j0 + Body::kFold));
         }
       }
     }

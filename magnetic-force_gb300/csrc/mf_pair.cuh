@@ -471,28 +471,20 @@ __device__ __forceinline__ void force_near_pq_rn(float r2, const float* __restri
   Q = fmaf(-3.f, c1, c2) * s * (ri * ri);
 }
 
-// (P, Q) of the force tensor for any pair, FP32 (k.tbl set).  A branch, not a
-// select: the external dipoles and the probe points this serves are mostly
-// farther than 4h from every source, and a warp whose lanes all are skips the
-// curves.
-__device__ __forceinline__ void force_coeffs_near_far(float r2, const PairConsts<float>& k, float& P, float& Q) {
-  const float ri = rsqrt_approx(r2), ri2 = ri * ri;
-  P = ri2 * ri2 * ri;
-  Q = -5.f * P * ri2;
-  if (r2 <= k.near2_force) {
-    P = Q = 0.f;
-    if (r2 > 0.f) force_near_pq_rn(r2, k.tbl, k.inv_h, k.ih4_over_k, P, Q);
-  }
+// (P, Q) of the force tensor for any pair, FP32 without a branch (k.tbl set).
+__device__ __forceinline__ void force_coeffs_sel(float r2, const PairConsts<float>& k, float& P, float& Q) {
+  float Pn, Qn;
+  force_near_pq_rn(r2, k.tbl, k.inv_h, k.ih4_over_k, Pn, Qn);
+  const float ri = rsqrt_approx(r2), ri2 = ri * ri, ri5 = ri2 * ri2 * ri;
+  const bool far = r2 > k.near2_force, apart = r2 > 0.f;
+  P = far ? ri5 : apart ? Pn : 0.f;
+  Q = far ? -5.f * ri5 * ri2 : apart ? Qn : 0.f;
 }
 
 // One tensor pair (6 unique entries xx, yy, zz, xy, xz, yz): t += T(d, s) / K.
 template <class Real>
-__device__ __forceinline__ void tensor_pair(Real dx, Real dy, Real dz, Real sx, Real sy, Real sz,
-                                            const PairConsts<Real>& k, Real* t) {
-  Real r2 = dx * dx + dy * dy + dz * dz;
-  Real P, Q;
-  if constexpr (sizeof(Real) == 4) force_coeffs_near_far(r2, k, P, Q);
-  else force_coeffs(r2, k, P, Q);
+__device__ __forceinline__ void tensor_terms(Real dx, Real dy, Real dz, Real sx, Real sy, Real sz, Real P, Real Q,
+                                             Real* t) {
   Real ds = dx * sx + dy * sy + dz * sz;
   Real pd = P * ds, qd = Q * ds;
   Real ax = P * sx, ay = P * sy, az = P * sz;
@@ -502,6 +494,15 @@ __device__ __forceinline__ void tensor_pair(Real dx, Real dy, Real dz, Real sx, 
   t[3] += ax * dy + ay * dx + qd * dx * dy;
   t[4] += ax * dz + az * dx + qd * dx * dz;
   t[5] += ay * dz + az * dy + qd * dy * dz;
+}
+template <class Real>
+__device__ __forceinline__ void tensor_pair(Real dx, Real dy, Real dz, Real sx, Real sy, Real sz,
+                                            const PairConsts<Real>& k, Real* t) {
+  Real r2 = dx * dx + dy * dy + dz * dz;
+  Real P, Q;
+  if constexpr (sizeof(Real) == 4) force_coeffs_sel(r2, k, P, Q);
+  else force_coeffs(r2, k, P, Q);
+  tensor_terms<Real>(dx, dy, dz, sx, sy, sz, P, Q, t);
 }
 
 }  // namespace mfgb
