@@ -121,7 +121,8 @@ __global__ void k_fmm_count(const float4* __restrict__ pos, int64_t n, FmmLevel 
 
 // Exclusive scan of the even-padded counts into start[0..n], one CTA.
 __global__ void __launch_bounds__(1024) k_fmm_scan(const int32_t* __restrict__ cnt, int64_t n,
-                                                   int32_t* __restrict__ start) {
+                                                   int32_t* __restrict__ start, int32_t* __restrict__ extra_n) {
+  if (extra_n && threadIdx.x == 0) *extra_n = 0;
   __shared__ int32_t sh[1024];
   const int t = threadIdx.x;
   const int64_t chunk = (n + 1023) / 1024;
@@ -151,9 +152,12 @@ __global__ void k_fmm_scatter(const int32_t* __restrict__ cell_of, int64_t n, in
 }
 
 // Each box's list in increasing particle index (one warp per box ranks its
-// entries), then -1 in the padding slot of an odd box.
+// entries), then -1 in the padding slot of an odd box.  extra (optional): (box,
+// first target) of every further run of `chunk` targets of a box, extra_n of
+// them, in any order (k_fmm_near_warp).
 __global__ void k_fmm_sort(const int32_t* __restrict__ start, const int32_t* __restrict__ cnt, int64_t ncell,
-                           const int32_t* __restrict__ tmp, int32_t* __restrict__ perm) {
+                           const int32_t* __restrict__ tmp, int32_t* __restrict__ perm, int32_t chunk,
+                           int2* __restrict__ extra, int32_t* __restrict__ extra_n) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
   for (int64_t c = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ncell; c += warps) {
@@ -165,6 +169,13 @@ __global__ void k_fmm_sort(const int32_t* __restrict__ start, const int32_t* __r
       perm[b + rank] = v;
     }
     if (lane == 0 && (m & 1)) perm[b + m] = -1;
+    if (extra && m > chunk) {
+      const int32_t runs = (m - 1) / chunk;
+      int32_t at = 0;
+      if (lane == 0) at = atomicAdd(extra_n, runs);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      for (int32_t k = lane; k < runs; k += 32) extra[at + k] = make_int2(int(c), (k + 1) * chunk);
+    }
   }
 }
 
@@ -655,6 +666,10 @@ struct P2PArgs {
   int32_t n_hrows;
   const float* part;
   int64_t n_slots;
+  // k_fmm_near_warp: targets of a CTA, and the runs beyond a box's first.
+  int32_t n_boxes, chunk;
+  const int2* extra;
+  const int32_t* extra_n;
 };
 
 // Plane of box offset dx in half row hr (1 + offsets before the row + index).
@@ -918,8 +933,8 @@ __global__ void __launch_bounds__(TPB) k_fmm_p2p(const P2PArgs p, const AllPairs
 // the record loads behind them: 8 bytes from L1 or L2 per pair (LSU wavefronts
 // 49 %), which is why big boxes in great number stay with the staged kernel
 // (launch_near).  Unrolling the item loop loses 8 % at 330,000 particles.
-// Whole step of 200,003 particles (boxes of ~20) 13.69 -> 11.57 ms, of 330,000
-// (few boxes of ~155) 29.86 -> 23.78, field product of 150,000 sources at
+// Whole step of a sphere of 200,003 particles (76 per occupied box) 13.69 -> 11.57
+// ms, of 330,000 (124) 29.86 -> 23.78, field product of 150,000 sources at
 // 30,011 separate targets 1.97 -> 1.32 ms, tensor 3.89 -> 2.68.  Other splits of the
 // 32 lanes (targets per lane x lane groups), the same step at 200,003: 4 x 16
 // 12.31, 4 x 8 12.58, 2 x 16 11.99, 8 x 32 12.69, 2 x 4 14.33 ms.
@@ -927,6 +942,7 @@ __global__ void __launch_bounds__(TPB) k_fmm_p2p(const P2PArgs p, const AllPairs
 constexpr int kNearT = 4;         // targets of a round
 constexpr int kNearFold = 64;     // items of a lane between folds of its FP32 sums
 constexpr int kNearMaxWarps = 8;  // warps per CTA (one box), taking rounds in turn
+constexpr int kNearRounds = 4;    // rounds of a warp; a box's further targets go to further CTAs
 template <int Q>
 struct NearWarp {
   static constexpr int kHead = (ncoef(Q) - 1 + 3) & ~3;       // words per CTA: the box's locals
@@ -945,8 +961,15 @@ __global__ void __launch_bounds__(32 * kNearMaxWarps, 2)
   extern __shared__ __align__(16) float near_smem[];
   if (p.done && *p.done != 0.0) return;
   const FmmLevel& lv = p.lv;
-  const int64_t c = blockIdx.x;
-  const int32_t n = p.tcnt[c];
+  int64_t c = blockIdx.x;
+  int32_t first = 0;
+  if (c >= p.n_boxes) {
+    const int64_t e = c - p.n_boxes;
+    if (e >= *p.extra_n) return;
+    c = p.extra[e].x;
+    first = p.extra[e].y;
+  }
+  const int32_t n = min(p.tcnt[c], first + p.chunk);
   if (n == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int ix = int(c % lv.nx), iy = int((c / lv.nx) % lv.ny), iz = int(c / (int64_t(lv.nx) * lv.ny));
@@ -957,7 +980,7 @@ __global__ void __launch_bounds__(32 * kNearMaxWarps, 2)
   float* pw = ws + 64;                        // [3 Q][kNearT]
   for (int k = threadIdx.x; k < ncoef(Q) - 1; k += blockDim.x) s_L[k] = p.L[int64_t(k) * lv.nbox + c];
   __syncthreads();  // the only block barrier: the warps part ways here
-  for (int t0 = warp * kNearT; t0 < n; t0 += nw * kNearT) {
+  for (int t0 = first + warp * kNearT; t0 < n; t0 += nw * kNearT) {
     typename Body::TData td[kNearT];
     float run[kNearT][kOut], cmp[kNearT][kOut];
 #pragma unroll
@@ -1547,12 +1570,19 @@ mf_status Fmm::build(const float4* pos4, int64_t n, const float4* tpos4, int64_t
   MF_TRY(perm_.reserve_slack(size_t(n + ncell + 2) * sizeof(int32_t)));
   MF_CUDA_TRY(cudaMemsetAsync(cnt, 0, size_t(ncell) * sizeof(int32_t), st));
   k_fmm_count<<<blocks_for(n), 256, 0, st>>>(pos4, n, leaf, cell_of_.as<int32_t>(), cnt);
-  k_fmm_scan<<<1, 1024, 0, st>>>(cnt, ncell, start_.as<int32_t>());
+  // Warps per box and targets per CTA of the near field, and its list of runs.
+  near_warps_ = int(std::min<int64_t>(kNearMaxWarps, (nt_ + ncell * kNearT - 1) / (ncell * kNearT)));
+  near_chunk_ = near_warps_ * kNearT * kNearRounds;
+  MF_TRY(extra_.reserve_slack(sizeof(int2) * size_t(1 + nt_ / near_chunk_) + 16));
+  int32_t* extra_n = extra_.as<int32_t>();
+  int2* extra = reinterpret_cast<int2*>(extra_.as<char>() + 16);
+  k_fmm_scan<<<1, 1024, 0, st>>>(cnt, ncell, start_.as<int32_t>(), separate_ ? nullptr : extra_n);
   MF_CUDA_TRY(cudaMemcpyAsync(cursor_.ptr, start_.ptr, size_t(ncell) * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
   k_fmm_scatter<<<blocks_for(n), 256, 0, st>>>(cell_of_.as<int32_t>(), n, cursor_.as<int32_t>(),
                                                 perm_tmp_.as<int32_t>());
   k_fmm_sort<<<blocks_for(ncell * 32), 256, 0, st>>>(start_.as<int32_t>(), cnt, ncell, perm_tmp_.as<int32_t>(),
-                                                      perm_.as<int32_t>());
+                                                      perm_.as<int32_t>(), near_chunk_, separate_ ? nullptr : extra,
+                                                      extra_n);
   for (int l = L - 1; l >= 0; --l)
     k_fmm_occ_up<<<blocks_for(lv_[size_t(l)].nbox), 256, 0, st>>>(lv_[size_t(l + 1)], lv_[size_t(l)], occ);
   MF_CUDA_TRY(cudaGetLastError());
@@ -1569,13 +1599,13 @@ mf_status Fmm::build(const float4* pos4, int64_t n, const float4* tpos4, int64_t
     MF_TRY(tperm_.reserve_slack(size_t(nt + ncell + 2) * sizeof(int32_t)));
     MF_CUDA_TRY(cudaMemsetAsync(tcnt, 0, size_t(ncell) * sizeof(int32_t), st));
     k_fmm_count<<<blocks_for(nt), 256, 0, st>>>(tpos4, nt, leaf, tcell_of_.as<int32_t>(), tcnt);
-    k_fmm_scan<<<1, 1024, 0, st>>>(tcnt, ncell, tstart_.as<int32_t>());
+    k_fmm_scan<<<1, 1024, 0, st>>>(tcnt, ncell, tstart_.as<int32_t>(), extra_n);
     MF_CUDA_TRY(cudaMemcpyAsync(tcursor_.ptr, tstart_.ptr, size_t(ncell) * sizeof(int32_t), cudaMemcpyDeviceToDevice,
                                 st));
     k_fmm_scatter<<<blocks_for(nt), 256, 0, st>>>(tcell_of_.as<int32_t>(), nt, tcursor_.as<int32_t>(),
                                                    tperm_tmp_.as<int32_t>());
     k_fmm_sort<<<blocks_for(ncell * 32), 256, 0, st>>>(tstart_.as<int32_t>(), tcnt, ncell, tperm_tmp_.as<int32_t>(),
-                                                        tperm_.as<int32_t>());
+                                                        tperm_.as<int32_t>(), near_chunk_, extra, extra_n);
     for (int l = L - 1; l >= 0; --l)
       k_fmm_occ_up<<<blocks_for(lv_[size_t(l)].nbox), 256, 0, st>>>(lv_[size_t(l + 1)], lv_[size_t(l)], tocc);
     MF_CUDA_TRY(cudaGetLastError());
@@ -1711,25 +1741,29 @@ mf_status Fmm::product(int kind, const float4* pos4, const float4* smom, const A
 
 namespace {
 // The near field of a product: four targets per warp (k_fmm_near_warp), as many
-// warps per box as a mean box has rounds, up to eight (steps at 200,003
-// particles, boxes of 16 on average: 2-4 warps 11.6-11.7 ms, 8 12.1; at
-// 330,000, few boxes of 81: 2 warps 28.6, 8 23.8).  The staged CTA of 128 targets
-// per box (k_fmm_p2p) is kept for the field where there are many boxes whose
-// targets nearly fill it: at 1,048,576 particles (12,800 boxes of 82 on
-// average) the step takes 54.4 ms with it against 55.7, while at 800,000 (62) it
-// takes 43.3 against 41.2 and in 4,074 boxes of 81 29.9 against 23.8.
+// warps per CTA as a mean box has rounds, up to eight (steps of a sphere of
+// 200,003 particles, 49 per box: 2-4 warps 11.6-11.7 ms, 8 12.1; of 330,000, 81
+// per box: 2 warps 28.6, 8 23.8).  A CTA takes four rounds of its warps, a
+// fuller box goes over several: the mean counts empty boxes and says nothing of
+// boxes that hold many targets (10,000 targets in one box of 150,000 sources: 39
+// ms for the field where one warp walked them all, 7.1 by 128-target CTAs, 0.49
+// now; on a line 9.6, 3.6, 0.82; spread evenly 0.88).
+// The staged CTA of 128 targets per box (k_fmm_p2p) is kept for the field of a
+// set on itself where there are many boxes that fill it.  Near fields, staged /
+// warps: 12,800 boxes of 82 (1,048,576 particles) 54.4 / 55.7 ms for the step,
+// 800,000 (62) 43.3 / 41.2, a sphere of 330,000 (4,074 of 81) 29.9 / 23.8 ms.
 template <int Q, int kKind>
-void launch_near(unsigned boxes, int64_t nt, cudaStream_t st, const P2PArgs& pp, const AllPairsArgs<float>& a,
+void launch_near(unsigned boxes, int64_t nt, bool separate, int warps, cudaStream_t st, const P2PArgs& pp, const AllPairsArgs<float>& a,
                  const SceneDesc<float>& sc) {
   if constexpr (kKind == 0) {
-    if (boxes >= 8192 && nt > 64 * int64_t(boxes) && nt <= 128 * int64_t(boxes)) {
+    const int64_t b = boxes;
+    if (!separate && b >= 8192 && nt > 64 * b && nt <= 128 * b) {
       k_fmm_p2p<Q, 0, false, 128, 256><<<boxes, 128, p2p_smem<256>(), st>>>(pp, a, sc);
       return;
     }
   }
-  const int64_t rounds = (nt + int64_t(boxes) * kNearT - 1) / (int64_t(boxes) * kNearT);
-  const int warps = int(std::min<int64_t>(kNearMaxWarps, std::max<int64_t>(1, rounds)));
-  k_fmm_near_warp<Q, kKind><<<boxes, 32 * warps, NearWarp<Q>::smem(warps), st>>>(pp, a, sc);
+  const unsigned ctas = boxes + unsigned(nt / pp.chunk);  // the extra runs are at most so many
+  k_fmm_near_warp<Q, kKind><<<ctas, 32 * warps, NearWarp<Q>::smem(warps), st>>>(pp, a, sc);
 }
 }  // namespace
 
@@ -1814,6 +1848,10 @@ mf_status Fmm::product_q(int kind, const float4* pos4, const float4* smom, const
   pp.rows = rows_.as<int4>();
   pp.n_rows = n_rows_;
   pp.done = done;
+  pp.n_boxes = int32_t(leaf.nbox);
+  pp.chunk = near_chunk_;
+  pp.extra_n = extra_.as<int32_t>();
+  pp.extra = reinterpret_cast<const int2*>(extra_.as<char>() + 16);
   const bool sym = kind == 1 && sym_near && !separate_;
   if (sym) {
     MF_TRY(npart_.reserve_grow(size_t(1 + n_off_) * 3 * size_t(n_slots_) * sizeof(float)));
@@ -1844,11 +1882,11 @@ mf_status Fmm::product_q(int kind, const float4* pos4, const float4* smom, const
     ++nl;
     k_fmm_p2p<Q, 1, true, 128, 256><<<unsigned(leaf.nbox), 128, p2p_smem<256>(), st>>>(pp, a, sc);
   } else if (kind == 1)
-    launch_near<Q, 1>(unsigned(leaf.nbox), nt_, st, pp, a, sc);
+    launch_near<Q, 1>(unsigned(leaf.nbox), nt_, separate_, near_warps_, st, pp, a, sc);
   else if (kind == 2)
-    launch_near<Q, 2>(unsigned(leaf.nbox), nt_, st, pp, a, sc);
+    launch_near<Q, 2>(unsigned(leaf.nbox), nt_, separate_, near_warps_, st, pp, a, sc);
   else
-    if constexpr (Q <= kMaxFieldDegree) launch_near<Q, 0>(unsigned(leaf.nbox), nt_, st, pp, a, sc);
+    if constexpr (Q <= kMaxFieldDegree) launch_near<Q, 0>(unsigned(leaf.nbox), nt_, separate_, near_warps_, st, pp, a, sc);
   ++nl;
   if (marks) MF_CUDA_TRY(cudaEventRecord(marks[3], st));
   launches_ = nl;
