@@ -1751,13 +1751,15 @@ namespace {
 // The staged CTA of 128 targets per box (k_fmm_p2p) is kept for the field of a
 // set on itself where there are many boxes that fill it.  Near fields, staged /
 // warps: 12,800 boxes of 82 (1,048,576 particles) 54.4 / 55.7 ms for the step,
-// 800,000 (62) 43.3 / 41.2, a sphere of 330,000 (4,074 of 81) 29.9 / 23.8 ms.
+// 800,000 (62) 43.3 / 41.2, a sphere of 330,000 (4,074 of 81) 29.9 / 23.8;
+// 4,096 boxes of 244 27.2 / 27.2, of 488 98.5 / 104.0, of 977 385 / 412, 512
+// boxes of 977 54.0 / 40.4 ms.
 template <int Q, int kKind>
 void launch_near(unsigned boxes, int64_t nt, bool separate, int warps, cudaStream_t st, const P2PArgs& pp, const AllPairsArgs<float>& a,
                  const SceneDesc<float>& sc) {
   if constexpr (kKind == 0) {
     const int64_t b = boxes;
-    if (!separate && b >= 8192 && nt > 64 * b && nt <= 128 * b) {
+    if (!separate && ((b >= 8192 && nt > 64 * b && nt <= 128 * b) || (b >= 4096 && nt > 256 * b))) {
       k_fmm_p2p<Q, 0, false, 128, 256><<<boxes, 128, p2p_smem<256>(), st>>>(pp, a, sc);
       return;
     }
