@@ -933,8 +933,8 @@ __global__ void __launch_bounds__(TPB) k_fmm_p2p(const P2PArgs p, const AllPairs
 // the record loads behind them: 8 bytes from L1 or L2 per pair (LSU wavefronts
 // 49 %), which is why big boxes in great number stay with the staged kernel
 // (launch_near).  Unrolling the item loop loses 8 % at 330,000 particles.
-// Whole step of a sphere of 200,003 particles (76 per occupied box) 13.69 -> 11.57
-// ms, of 330,000 (124) 29.86 -> 23.78, field product of 150,000 sources at
+// Whole step of a cylinder of 200,003 particles (16 per box) 13.69 -> 11.57 ms, of
+// a sphere of 330,000 (81, 124 per occupied box) 29.86 -> 23.78, field product of 150,000 sources at
 // 30,011 separate targets 1.97 -> 1.32 ms, tensor 3.89 -> 2.68.  Other splits of the
 // 32 lanes (targets per lane x lane groups), the same step at 200,003: 4 x 16
 // 12.31, 4 x 8 12.58, 2 x 16 11.99, 8 x 32 12.69, 2 x 4 14.33 ms.
@@ -1741,9 +1741,9 @@ mf_status Fmm::product(int kind, const float4* pos4, const float4* smom, const A
 
 namespace {
 // The near field of a product: four targets per warp (k_fmm_near_warp), as many
-// warps per CTA as a mean box has rounds, up to eight (steps of a sphere of
-// 200,003 particles, 49 per box: 2-4 warps 11.6-11.7 ms, 8 12.1; of 330,000, 81
-// per box: 2 warps 28.6, 8 23.8).  A CTA takes four rounds of its warps, a
+// warps per CTA as a mean box has rounds, up to eight (steps of a cylinder of
+// 200,003 particles, 16 per box: 2-4 warps 11.6-11.7 ms, 8 12.1; of a sphere of
+// 330,000, 81 per box: 2 warps 28.6, 8 23.8).  A CTA takes four rounds of its warps, a
 // fuller box goes over several: the mean counts empty boxes and says nothing of
 // boxes that hold many targets (10,000 targets in one box of 150,000 sources: 39
 // ms for the field where one warp walked them all, 7.1 by 128-target CTAs, 0.49
