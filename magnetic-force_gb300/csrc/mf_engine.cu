@@ -681,6 +681,21 @@ class Engine final : public EngineBase {
 
   double c_coef() const { return double(volume_) * double(chi_) / (double(chi_) + 1.0); }
 
+  // Whether the force takes the packed kernels (kPackedForceMin).  Near pairs
+  // per particle: what its volume says, or the bounding box where that is less.
+  mf_status force_packed(bool* yes) {
+    *yes = kF32 && np_ >= kPackedForceMin;
+    if constexpr (kF32) {
+      if (!*yes || np_ >= kPackedForceAlways || sym_mode_ == 2) return MF_OK;
+      MF_TRY(ensure_cells());
+      double box = 1.0;
+      for (int k = 0; k < 3; ++k) box *= cells_.bbox(0)[3 + k] - cells_.bbox(0)[k] + std::cbrt(volume_);
+      const double ball = 4.0 / 3.0 * kPi * 64.0 * h_ * h_ * h_;
+      *yes = ball <= kPackedForceNear * std::min(volume_, box / double(np_));
+    }
+    return MF_OK;
+  }
+
   mf_status build_plans() {
     const double c = c_coef();
     SceneSpec base;
@@ -696,7 +711,9 @@ class Engine final : public EngineBase {
     s.coef_add2 = -1.0;
     // FP32 uses the packed two-source kernels; FP64 the exact-branch kernels.
     const Body fb = (kF32 && np_ >= kPackedFieldMin) ? Body::FieldF2 : Body::Field;
-    const Body gb = (kF32 && np_ >= kPackedForceMin) ? Body::ForceF2 : Body::Force;
+    bool packed_force = false;
+    MF_TRY(force_packed(&packed_force));
+    const Body gb = packed_force ? Body::ForceF2 : Body::Force;
     // FP32: block shapes from the autotuner, timed on this scene's own
     // positions (the tuning launches write scratch vectors only).
     // The packed products may run once per unordered pair (kShapeSym): the

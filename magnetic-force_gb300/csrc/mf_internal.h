@@ -108,9 +108,15 @@ enum class Body { Field = 0, Force = 1, Tensor = 2, FieldF2 = 3, ForceF2 = 4, Te
 // Force, one scene alone (whole steps, exact against packed): 404 / 449 us at
 // 6,000 particles, 519 / 523 at 8,000, 638 / 605 at 10,000, 756 / 699 at
 // 12,289.  (Before the correction took two targets per instruction the line
-// lay at 14,336.)
+// lay at 14,336.)  That is at h = 2 spacings, 2,145 particles inside 4h.  The
+// correction grows with these and the exact kernels do not: forces at h = 2,
+// 2.25, 2.5 and 4 spacings, packed (exact the same at all), 222 / 274 / 337 / 636
+// (219) us at 8,192, 334 / 384 / 497 / 981 (393) at 12,289, 435 / 495 / 560 /
+// 1,197 (577) at 14,335.  So below 14,336 only where at most 2,300 are expected.
 constexpr int64_t kPackedFieldMin = 2048;
 constexpr int64_t kPackedForceMin = 8192;
+constexpr int64_t kPackedForceAlways = 14336;
+constexpr double kPackedForceNear = 2300.0;
 // Force inside a batch: one packed launch and one correction launch serve all
 // large scenes, so the packed path wins from smaller scenes on (256 scenes of
 // 512..32,768 particles: 92.2 ms per step at 12,288, 89.7 ms at 4,096; 64 of
