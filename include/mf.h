@@ -113,7 +113,8 @@ typedef enum mf_option {
                                each unordered pair evaluated once for both particles (a pair
                                kernel and a per-particle finish) instead of every ordered
                                pair: 0 never, 1 where tuning measured it faster (default;
-                               without tuning, the force only), 2 always.  FP64 handles of at
+                               without tuning, the force only,
+                               of a scene alone from 13,312 particles on), 2 always.  FP64 handles of at
                                most 65,536 particles have kernels of the same kind: 0 never,
                                1 and 2 always.  On the FMM path
                                the force's near field is evaluated once per unordered box

@@ -566,7 +566,10 @@ std::atomic<uint32_t> g_stage_wait_debug{0};
 uint32_t stage_wait_debug() { return g_stage_wait_debug.load(std::memory_order_relaxed); }
 void set_stage_wait_debug(uint32_t v) { g_stage_wait_debug.store(v, std::memory_order_relaxed); }
 
+// Without tuning the force runs once per unordered pair, except for one scene of
+// few block pairs (kSymDefaultMin).
 int default_shape(Body body, const std::vector<SceneSpec>& specs, bool allow_sym) {
+  if (specs.size() == 1 && specs[0].nt < kSymDefaultMin) return 0;
   return allow_sym && body == Body::ForceF2 && sym_eligible(body, specs) ? kShapeSym : 0;
 }
 

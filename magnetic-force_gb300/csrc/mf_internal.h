@@ -127,6 +127,11 @@ constexpr int64_t kBatchPackedForceMin = 4096;
 // particles: force 0.82 against 1.04 ms; at 16,384 the all-pairs field wins
 // (0.206 against 0.213 ms).
 constexpr int64_t kSymDirectMin = 32768;
+// One scene without tuning: the force once per unordered pair from this size on.
+// Blocks of 1,024 give 36 steps to 304 CTAs at 8,192 particles: forces 347 us
+// against 224 by all pairs there, 361 / 273 at 10,000, 375 / 347 at 12,289, 398 /
+// 421 at 14,000.
+constexpr int64_t kSymDefaultMin = 13312;
 // FMM handles: the force's near field once per unordered box pair from this
 // size on.  Measured when the force's aperture was 0.3 (its half stencil ~4x
 // the partial-sum planes of 0.5): force products on the r = 0.3 cylinder
