@@ -116,7 +116,8 @@ typedef enum mf_option {
                                without tuning, the force only,
                                of a scene alone from 13,312 particles on), 2 always.  FP64 handles of at
                                most 65,536 particles have kernels of the same kind: 0 never,
-                               1 and 2 always.  On the FMM path
+                               1 and 2 always where their block sums (0.4 GB at 65,536) can be
+                               allocated.  On the FMM path
                                the force's near field is evaluated once per unordered box
                                pair with 2, and with 1 from 1,048,576 particles on.  Not in
                                the reference. */

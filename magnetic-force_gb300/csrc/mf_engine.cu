@@ -759,6 +759,15 @@ class Engine final : public EngineBase {
       if (sym64_eligible(gb, {base})) gshape = kShapeSym;
     }
     MF_TRY(build_plan<Real>(fb, {s}, plan_resid_, fshape));
+    if constexpr (!kF32) {
+      // Its block sums take up to 0.4 GB (24 n^2 bytes over the block size); where
+      // they cannot be had, all pairs, which need next to nothing.
+      if (fshape == kShapeSym && scr_.ensure(sym64_partials(plan_resid_), 0) != MF_OK) {
+        cudaGetLastError();
+        fshape = gshape = 0;
+        MF_TRY(build_plan<Real>(fb, {s}, plan_resid_, fshape));
+      }
+    }
     // gradient g = c G(r) - r            (D_transpose, :1281-1284)
     // D(d) = c G(d) - d                  (D, :1275-1278)
     s = base;
