@@ -1637,7 +1637,14 @@ mf_status Fmm::build(const float4* pos4, int64_t n, const float4* tpos4, int64_t
       const double r0 = std::sqrt(double(d2));
       return cfg.theta * r0 > r12 && (r0 - r12) * s > rnear;
     };
+    // No two boxes are as far apart as kNoFar: beyond, nothing is far (and the
+    // square of a radius at a tiny theta need not fit).
+    constexpr double kNoFar = double(2 << kMaxLevel);
     const double t = std::max(r12 / cfg.theta, r12 + rnear / s);
+    if (!(t < kNoFar)) {
+      m[size_t(l)] = int64_t(kNoFar * kNoFar);
+      continue;
+    }
     int64_t d2 = int64_t(t * t);
     while (d2 > 0 && is_far(d2)) --d2;
     while (!is_far(d2 + 1)) ++d2;
