@@ -1,29 +1,33 @@
 // mf_sym64.cu -- the FP64 field and force products evaluated once per
 // unordered pair of particles.
 //
-// GB300 issues fewer than two FP64 operations per SM and clock, 1/64 of its FP32
+// GB300 issues two FP64 operations per SM and clock, 1/64 of its FP32
 // rate, so the FP64 instructions are all that counts here: loads, shuffles,
 // integer work and selects ride along free.  The kernels below spend as few
 // of them as the exact pair terms allow:
 //   * both terms of a pair come from one evaluation (the field tensor is even
 //     in d, the Kelvin force odd; see mf_sympair.cu);
-//   * no square root and no division: a hardware seed y of r^-1 (~20 bits)
-//     and e = 1 - r^2 y^2 give r^-3 = y^3 (1 + 3/2 e + 15/8 e^2), r^-5 and
-//     r^-2 by their binomial series, the terms left out below 2^-56;
+//   * no square root and no division: a hardware seed y of r^-1 and e = 1 -
+//     r^2 y^2, at most 2^-19.04 (measured over r^2 in [1, 4)), give r^-3 = y^3
+//     (1 + 3/2 e + 15/8 e^2), r^-5 and r^-2 by their binomial series; the first
+//     terms left out, 35/16 e^3, 105/16 e^3 and e^3, are at most 2^-56.0, 2^-54.4
+//     and 2^-57.1;
 //   * the near forms (SPH weights inside 2h, fitted curves inside 4h) are
 //     polynomials in q with coefficients looked up per lane, evaluated where
 //     any lane of the warp needs them, and selected;
 //   * each lane holds one target and meets the 32 sources of a sub-tile in
 //     rotation, the sources' sums travelling from lane to lane, so no sum
 //     needs a reduction tree.
-// Per unordered pair the field takes 35 FP64 operations (47 with a near lane
-// in the warp), the force 46 (66).  Measured at 4,096 uniformly random
-// particles, where most warps have a near lane at every rotation: field
-// product 0.66 ms against 3.01 for the all-pairs kernel (~105 operations per
+// Per unordered pair the field takes 36 FP64 operations, comparisons included
+// (50 with a near lane in the warp), the force 47 (72).  At 4,096 uniformly random
+// particles 79 % of the rotations have a near lane for the field, all for the
+// force: 47 and 72 operations, 0.64 and 0.97 ms of the FP64 units at their nominal
+// rate (a warp's operation 16 cycles of an SM).  Measured with the finish: field
+// product 0.80 ms against 3.0 for the all-pairs kernel (~105 operations per
 // ordered pair: both branches with their square roots and divisions), force
-// 1.20 against 3.21.  A warp's FP64 operation takes 76 cycles of its SM
-// quarter (19 per SM, measured), so 0.66 ms is the FP64 units' rate: what is
-// left is the operation count.
+// 1.21 against 3.2.  The FP64 units bound both; what is left is the operation count
+// and a chain of dependent operations at 61 cycles each (measured 19 cycles of an
+// SM per operation in place of 16).
 //
 // Work layout: blocks of TB = 32 W particles (W warps per CTA), steps = block
 // pairs (I, J), I <= J, split evenly over the resident CTAs; every step writes
@@ -257,28 +261,37 @@ __global__ void __launch_bounds__(32 * W) k_sym64(const Sym64Args p) {
       __syncthreads();
       Vec3d src{0.0, 0.0, 0.0};  // the sums of source (lane + r) & 31 at rotation r
       const bool sym = I != J;   // block-uniform
-      // A block with itself hands nothing on: its live sources in turn (32
-      // rotations take 80 us however few there are: forces of 1 and 10 particles
-      // 118 us against 43 and 66 by all pairs, 41 and 61 this way).
-      const int64_t live = p.n - (int64_t(J) * TB + h * 32);
-      const int n_rot = sym ? 32 : int(live < 32 ? (live < 0 ? 0 : live) : 32);
+      if (sym) {
 #pragma unroll 1
-      for (int r = 0; r < n_rot; ++r) {
-        const int j = sym ? (lane + r) & 31 : r;
-        const Vec3d s{s_p[0][j], s_p[1][j], s_p[2][j]}, sm{s_m[0][j], s_m[1][j], s_m[2][j]};
-        if constexpr (kForce) {
-          if (sym) pair64_force<true>(t, tm, s, sm, pc, s_tbl, acc, src);
-          else pair64_force<false>(t, tm, s, sm, pc, s_tbl, acc, src);
-        } else {
-          const Vec3d sm3{s_m3[0][j], s_m3[1][j], s_m3[2][j]};
-          if (sym) pair64_field<true>(t, tm, tm3, s, sm, sm3, pc, s_tbl, acc, src);
-          else pair64_field<false>(t, tm, tm3, s, sm, sm3, pc, s_tbl, acc, src);
-        }
-        if (sym) {  // hand the sums to the lane that meets the source next
-          const int from = (lane + 1) & 31;
+        for (int r = 0; r < 32; ++r) {
+          const int j = (lane + r) & 31;
+          const Vec3d s{s_p[0][j], s_p[1][j], s_p[2][j]}, sm{s_m[0][j], s_m[1][j], s_m[2][j]};
+          if constexpr (kForce) {
+            pair64_force<true>(t, tm, s, sm, pc, s_tbl, acc, src);
+          } else {
+            const Vec3d sm3{s_m3[0][j], s_m3[1][j], s_m3[2][j]};
+            pair64_field<true>(t, tm, tm3, s, sm, sm3, pc, s_tbl, acc, src);
+          }
+          const int from = (lane + 1) & 31;  // hand the sums to the lane that meets the source next
           src.x = __shfl_sync(0xffffffffu, src.x, from);
           src.y = __shfl_sync(0xffffffffu, src.y, from);
           src.z = __shfl_sync(0xffffffffu, src.z, from);
+        }
+      } else {
+        // A block with itself hands nothing on: its live sources in turn (32
+        // rotations take 80 us however few there are: forces of 1 and 10
+        // particles 118 us against 43 and 66 by all pairs, 41 and 64 this way).
+        const int64_t live = p.n - (int64_t(J) * TB + h * 32);
+        const int n_src = live < 32 ? int(live < 0 ? 0 : live) : 32;
+#pragma unroll 1
+        for (int j = 0; j < n_src; ++j) {
+          const Vec3d s{s_p[0][j], s_p[1][j], s_p[2][j]}, sm{s_m[0][j], s_m[1][j], s_m[2][j]};
+          if constexpr (kForce) {
+            pair64_force<false>(t, tm, s, sm, pc, s_tbl, acc, src);
+          } else {
+            const Vec3d sm3{s_m3[0][j], s_m3[1][j], s_m3[2][j]};
+            pair64_field<false>(t, tm, tm3, s, sm, sm3, pc, s_tbl, acc, src);
+          }
         }
       }
       if (sym) {  // back at source `lane`
@@ -339,8 +352,8 @@ __global__ void __launch_bounds__(256) k_sym64_finish(const Sym64Args p, int tb)
 }
 
 // Warps per CTA: the finest split, one 32-particle block pair per warp, keeps
-// the four FP64 units of every SM evenly loaded (field product at 4,096
-// particles: 0.66 ms with one warp per CTA, 0.71 with two); larger blocks keep
+// the four FP64 units of every SM evenly loaded (field kernel at 4,096
+// particles: 7 % slower with two); larger blocks keep
 // the partial sums (24 n^2 / TB bytes) of larger scenes small.  16 or 8 warps
 // per SM measure the same, 32 take 8 % longer (the steps no longer divide
 // evenly).  Also the scratch bound: see sym64_eligible.
