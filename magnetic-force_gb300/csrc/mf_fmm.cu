@@ -1565,17 +1565,19 @@ mf_status Fmm::build(const float4* pos4, int64_t n, const float4* tpos4, int64_t
   int32_t* cnt = occ + leaf.box_off;
   MF_TRY(cell_of_.reserve(size_t(n) * sizeof(int32_t)));
   MF_TRY(start_.reserve_slack(size_t(ncell + 1) * sizeof(int32_t)));
-  MF_TRY(cursor_.reserve_slack(size_t(ncell + 1) * sizeof(int32_t)));
+  // The list of runs lies behind the cursors (whole 16 bytes on): its count,
+  // then 16 bytes on the entries.
+  near_warps_ = int(std::min<int64_t>(kNearMaxWarps, (nt_ + ncell * kNearT - 1) / (ncell * kNearT)));
+  near_chunk_ = near_warps_ * kNearT * kNearRounds;
+  const size_t cursors = (size_t(ncell + 1) * sizeof(int32_t) + 15) / 16 * 16;
+  MF_TRY(cursor_.reserve_slack(cursors + 16 + sizeof(int2) * size_t(1 + nt_ / near_chunk_)));
+  extra_ = cursor_.as<char>() + cursors;
+  int32_t* extra_n = reinterpret_cast<int32_t*>(extra_);
+  int2* extra = reinterpret_cast<int2*>(extra_ + 16);
   MF_TRY(perm_tmp_.reserve_slack(size_t(n + ncell + 2) * sizeof(int32_t)));
   MF_TRY(perm_.reserve_slack(size_t(n + ncell + 2) * sizeof(int32_t)));
   MF_CUDA_TRY(cudaMemsetAsync(cnt, 0, size_t(ncell) * sizeof(int32_t), st));
   k_fmm_count<<<blocks_for(n), 256, 0, st>>>(pos4, n, leaf, cell_of_.as<int32_t>(), cnt);
-  // Warps per box and targets per CTA of the near field, and its list of runs.
-  near_warps_ = int(std::min<int64_t>(kNearMaxWarps, (nt_ + ncell * kNearT - 1) / (ncell * kNearT)));
-  near_chunk_ = near_warps_ * kNearT * kNearRounds;
-  MF_TRY(extra_.reserve_slack(sizeof(int2) * size_t(1 + nt_ / near_chunk_) + 16));
-  int32_t* extra_n = extra_.as<int32_t>();
-  int2* extra = reinterpret_cast<int2*>(extra_.as<char>() + 16);
   k_fmm_scan<<<1, 1024, 0, st>>>(cnt, ncell, start_.as<int32_t>(), separate_ ? nullptr : extra_n);
   MF_CUDA_TRY(cudaMemcpyAsync(cursor_.ptr, start_.ptr, size_t(ncell) * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
   k_fmm_scatter<<<blocks_for(n), 256, 0, st>>>(cell_of_.as<int32_t>(), n, cursor_.as<int32_t>(),
@@ -1681,8 +1683,8 @@ mf_status Fmm::build(const float4* pos4, int64_t n, const float4* tpos4, int64_t
     chunks_[size_t(l)] = int32_t(ch);
     lpart = std::max(lpart, ch * nharm(Q) * v.nbox);
   }
-  MF_TRY(mcoef_.reserve_slack(size_t(NC) * size_t(nbox_total) * sizeof(float)));
-  MF_TRY(hcoef_.reserve_slack(size_t(nharm(Q)) * size_t(nbox_total) * sizeof(float)));
+  MF_TRY(mcoef_.reserve_slack(size_t(NC + nharm(Q)) * size_t(nbox_total) * sizeof(float)));
+  hcoef_ = mcoef_.as<float>() + int64_t(NC) * nbox_total;
   MF_TRY(lcoef_.reserve_slack(size_t(NC) * size_t(nbox_total) * sizeof(float)));
   MF_TRY(lpart_.reserve_slack(size_t(lpart) * sizeof(float)));
 
@@ -1788,7 +1790,7 @@ mf_status Fmm::product_q(int kind, const float4* pos4, const float4* smom, const
   const int32_t* tocc = separate_ ? tocc_.as<int32_t>() : occ;
   constexpr int NH = nharm(Q);
   float* M = mcoef_.as<float>();
-  float* H = hcoef_.as<float>();  // multipoles with z <= 1
+  float* H = hcoef_;  // multipoles with z <= 1
   float* Lc = lcoef_.as<float>();
   int nl = 0;
   if (marks) MF_CUDA_TRY(cudaEventRecord(marks[0], st));
@@ -1859,8 +1861,8 @@ mf_status Fmm::product_q(int kind, const float4* pos4, const float4* smom, const
   pp.done = done;
   pp.n_boxes = int32_t(leaf.nbox);
   pp.chunk = near_chunk_;
-  pp.extra_n = extra_.as<int32_t>();
-  pp.extra = reinterpret_cast<const int2*>(extra_.as<char>() + 16);
+  pp.extra_n = reinterpret_cast<const int32_t*>(extra_);
+  pp.extra = reinterpret_cast<const int2*>(extra_ + 16);
   const bool sym = kind == 1 && sym_near && !separate_;
   if (sym) {
     MF_TRY(npart_.reserve_grow(size_t(1 + n_off_) * 3 * size_t(n_slots_) * sizeof(float)));

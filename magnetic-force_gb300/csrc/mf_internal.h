@@ -556,9 +556,10 @@ class Fmm {
   int n_hrows_ = 0, n_off_ = 0;  // half-stencil rows and their box offsets (sym_near)
   int launches_ = 0;
   DevBuf cell_of_, cnt_, start_, cursor_, perm_tmp_, perm_, pos2s_, mom2s_;
-  DevBuf occ_, mcoef_, hcoef_, lcoef_, lpart_, lists_, rows_, dtab_, stat_, lofs_;
+  DevBuf occ_, mcoef_, lcoef_, lpart_, lists_, rows_, dtab_, stat_, lofs_;
   DevBuf hrows_, npart_;  // half-stencil rows; near-field partial sums (sym_near)
-  DevBuf extra_;          // runs of targets beyond a box's first: their count, 16 bytes on (box, first target)
+  float* hcoef_ = nullptr;  // in mcoef_: the multipoles with z <= 1
+  char* extra_ = nullptr;   // in cursor_: runs of targets beyond a box's first, their count, 16 bytes on (box, first target)
   int32_t near_warps_ = 1, near_chunk_ = 1;
   // Separate targets: occupancy per level and leaf binning.
   DevBuf tocc_, tcell_of_, tstart_, tcursor_, tperm_tmp_, tperm_;
