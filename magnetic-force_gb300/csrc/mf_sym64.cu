@@ -25,9 +25,9 @@
 // rate (a warp's operation 16 cycles of an SM).  Measured with the finish: field
 // product 0.80 ms against 3.0 for the all-pairs kernel (~105 operations per
 // ordered pair: both branches with their square roots and divisions), force
-// 1.21 against 3.2.  The FP64 units bound both; what is left is the operation count
-// and a chain of dependent operations at 61 cycles each (measured 19 cycles of an
-// SM per operation in place of 16).
+// 1.21 against 3.2.  The FP64 pipe is active 88 and 85 % of the kernels' time
+// (conversions and selects of the tables are on it too): what is left is the
+// operation count.
 //
 // Work layout: blocks of TB = 32 W particles (W warps per CTA), steps = block
 // pairs (I, J), I <= J, split evenly over the resident CTAs; every step writes

@@ -2,7 +2,8 @@
 them: compared with calls of the same kind right beside them.
 
 Bounds: the work of the two sides differs by the stated factor; half as much
-again is allowed for launches and noise (the wrong kernel takes 1.7 times and more).
+again is allowed for launches and noise, three quarters for the dense sets, whose
+cell list is made before it is left (the wrong kernel took 3.4, 1.7 and 2 times).
 """
 import time
 
@@ -49,4 +50,4 @@ def test_tensor_of_dense_sources(mf, cuda):
     t, s, m = sets(cuda, 12000, 12000)
     whole = best(cuda, lambda: mf.direct_force_tensor(t, s, m, 0.4))
     less = best(cuda, lambda: mf.direct_force_tensor(t[:10000], s[:10000], m[:10000], 0.4))
-    assert whole < 1.5 * 1.44 * less
+    assert whole < 1.75 * 1.44 * less
