@@ -97,7 +97,7 @@ struct RecordItems {
   // Items of a tile summed in plain FP32 before they join the running sums.
   // Whole tiles of 256 gave direct fields of 1,000 and 9,000 particles 2.3e-7
   // and 2.2e-7 from FP64 where the packed body gives 1.5e-7 and 1.4e-7; now
-  // 1.2e-7 both, 5 % slower at 11,000.
+  // 1.2e-7 both, 2 % slower at 11,000.
   static constexpr int kFold = sizeof(Real) == 4 ? 64 : 128;
   static constexpr int kGroup = 1;  // items a body takes at once (group())
   static constexpr int kSources = 1;  // per item

@@ -1764,8 +1764,8 @@ namespace {
 // 4,096 boxes of 244 27.2 / 27.2, of 488 98.5 / 104.0, of 977 385 / 412, 512
 // boxes of 977 54.0 / 40.4 ms.
 template <int Q, int kKind>
-void launch_near(unsigned boxes, int64_t nt, bool separate, int warps, cudaStream_t st, const P2PArgs& pp, const AllPairsArgs<float>& a,
-                 const SceneDesc<float>& sc) {
+void launch_near(unsigned boxes, int64_t nt, bool separate, int warps, cudaStream_t st, const P2PArgs& pp,
+                 const AllPairsArgs<float>& a, const SceneDesc<float>& sc) {
   if constexpr (kKind == 0) {
     const int64_t b = boxes;
     if (!separate && ((b >= 8192 && nt > 64 * b && nt <= 128 * b) || (b >= 4096 && nt > 256 * b))) {
