@@ -640,7 +640,7 @@ void to_pairs(const float4* src, float4* dst, int64_t n, cudaStream_t st, const 
 }
 
 mf_status CellList::build(const float4* pos4, const std::vector<CellSceneSpec>& scenes, cudaStream_t st,
-                          double margin_h) {
+                          double margin_h, const std::function<bool(const double*)>& wanted) {
   const int ns = int(scenes.size());
   if (ns == 0) return fail(MF_ERR_INVALID_ARG, "cell list: no scenes");
   n_scenes_ = ns;
@@ -680,6 +680,7 @@ mf_status CellList::build(const float4* pos4, const std::vector<CellSceneSpec>& 
       ext[c] = std::max(0.0, double(ord2f(hb[6 * s + 3 + c])) + margin_h * h - lo[c]);
       if (!std::isfinite(lo[c]) || !std::isfinite(ext[c])) return fail(MF_ERR_INVALID_ARG, "non-finite positions");
     }
+    if (wanted && !wanted(host_bbox_.data() + 6 * size_t(s))) return MF_OK;
     // Cells a hair wider than h (about 8 particles at h = 2 spacings): a point
     // closer than 2h (4h) to a target then always lies within 2 (4) cells of
     // it, whatever the rounding of the cell map.

@@ -64,41 +64,46 @@ unsigned grid_for(int64_t n) {
 
 constexpr int kBodies = 6;
 
-// Whether a call's packed kernels beat the exact-branch ones.  They cost a cell
-// list over the sources (ten launches, a host round trip, then with the count)
-// and the near-field correction, a warp per target; they save about half of
-// every pair of the padded target blocks.  Whole calls, exact / packed us:
-//   field, 64 x 200,000 746 / 513, 1,000 x 40,000 295 / 352, 4,000 x 40,000
-//   474 / 327, 40,000 x 4,000 405 / 346, 200,000 x 1,000 399 / 562; of one set
-//   (the correction by cells) 8,500 219 / 234, 9,000 333 / 261.
-//   force of one set, 10,000 358 / 333-405, 11,500 494 / 386-473 (few to many
-//   near pairs).
+// Whether a call's packed kernels can beat the exact-branch ones.  They cost a
+// cell list over the sources (ten launches, a host round trip, then with the
+// count) and the near-field correction, a warp per target; they save about half
+// of every pair of the padded target blocks.  Whole calls, exact / packed us:
+//   field, 64 x 200,000 612 / 653, 64 x 1,000,000 1,165 / 976, 1,000 x 200,000 562 /
+//   531, 4,000 x 40,000 355 / 346, 40,000 x 4,000 312 / 300-516, 200,000 x 1,000 399
+//   / 562; of one set (the correction by cells) 9,500 249 / 274, 12,000 323 / 305.
+//   force of one set, 9,500 347 / 324-407, 12,000 471 / 366-518 (few to many near
+//   pairs).
 //   tensor, 256 x 1,000,000 898 / 1,208, 1,000 x 200,000 644 / 624, 1,000 x
 //   1,000,000 2,033 / 1,480, 2,000 x 40,000 433 / 442, 11,000 x 10,000 424 /
 //   418, 40,000 x 10,000 1,331 / 976, 1,000,000 x 1,000 3,119 / 5,115.
+double padded_pairs(Body body, int64_t nt, int64_t ns) {
+  const int64_t block = body == Body::Tensor ? 128 : 512;
+  return double((nt + block - 1) / block * block) * double(ns);
+}
 bool packed_pays(Body body, bool one_set, int64_t nt, int64_t ns) {
-  const double t = double(nt), s = double(ns);
-  auto padded = [&](int64_t block) { return double((nt + block - 1) / block * block) * s; };
-  if (body == Body::Tensor) return padded(128) >= 9e7 + 360.0 * s + 2450.0 * t;
-  if (one_set) return t * s >= (body == Body::Field ? 7.6e7 : 1.25e8);
-  return padded(512) >= 7.5e7 + 1000.0 * t;
+  const double t = double(nt), s = double(ns), pairs = padded_pairs(body, nt, ns);
+  if (body == Body::Tensor) return pairs >= 9e7 + 360.0 * s + 2450.0 * t;
+  if (one_set) return t * s >= 1.25e8;
+  return pairs >= 1.4e8 + 1000.0 * t;
 }
 
-// Where many pairs are near, the correction costs more than the packed kernel
-// saves.  near_part: the part of the sources expected within `reach` of a
-// target (bbox: theirs), from which on the exact kernel is taken.  12,000 x
-// 12,000 in the unit cube at h = 0.05, 0.1, 0.2, 0.4, exact / packed us: field
-// (2h: 0.4, 3, 27, 52 %) 309 / 285, 310 / 289, 312 / 1,007, 313 / 5,976; force
-// (4h: 3, 27, 52, 52 %) 482 / 379, 484 / 462, 484 / 1,428, 484 / 8,136; tensor
-// 458 / 366, 534 / 521, 542 / 874, 534 / 1,084.
-constexpr double kDenseField = 0.06, kDenseForce = 0.3;
-double near_part(const double* bbox, double reach) {
-  double f = kPi / 6.0;
-  for (int k = 0; k < 3; ++k) f *= std::min(1.0, 2.0 * reach / std::max(bbox[3 + k] - bbox[k], 1e-300));
-  return f;
-}
-bool dense(Body body, const double* bbox, double h) {
-  return body == Body::Field ? near_part(bbox, 2.0 * h) > kDenseField : near_part(bbox, 4.0 * h) > kDenseForce;
+// And whether they do, given the sources' bounding box: where many pairs are
+// near, the correction costs more than the packed kernel saves.  The part of the
+// sources expected within the near radius (2h field, 4h force and tensor) at
+// which both take the same time, in uniform cubes:
+//   field, one set: 0.04 at 12,000, 0.07 at 20,000, 0.09 at 40,000; separate: 0.03
+//   at 40,000 x 4,000 and 12,000 x 12,000, 0.12 at 20,000 x 100,000;
+//   force: 0.14 at 9,500, 0.24 at 12,000, 0.26 at 20,000, 0.39 at 40,000;
+//   tensor: 0.2 at 12,000, 0.4 at 20,000, 0.52 at 40,000, 0.27 at 40,000 x 4,000.
+// Beyond it packed fields lose most: 12,000 of one set at 0.52, exact / packed
+// 330 / 1,695 us, force 474 / 685, tensor 487 / 647.
+bool few_near(Body body, bool one_set, int64_t nt, int64_t ns, double h, const double* bbox) {
+  const double reach = body == Body::Field ? 2.0 * h : 4.0 * h, pairs = padded_pairs(body, nt, ns);
+  double near = kPi / 6.0;
+  for (int k = 0; k < 3; ++k) near *= std::min(1.0, 2.0 * reach / std::max(bbox[3 + k] - bbox[k], 1e-300));
+  if (body == Body::Tensor) return near <= 0.55 - 5e7 / pairs;
+  if (body == Body::Force) return near <= 0.38 - 2e7 / pairs;
+  return near <= (one_set ? 0.105 - 9e6 / pairs : std::max(0.02, 0.135 - 1.6e7 / pairs));
 }
 
 struct DirectCtx {
@@ -191,12 +196,11 @@ mf_status direct_impl(Body body, const float* targets, int64_t nt, const float* 
   Body launch_body = body;
   bool packed = large;
   if (packed) {
-    const mf_status built = c.cells.build(c.s4.as<float4>(), {CellSceneSpec{0, ns, double(h)}}, st);
+    auto wanted = [&](const double* bbox) { return packed = few_near(body, one_set, nt, ns, double(h), bbox); };
+    const mf_status built = c.cells.build(c.s4.as<float4>(), {CellSceneSpec{0, ns, double(h)}}, st, 0.0, wanted);
     if (built != MF_OK) {
       if (body != Body::Tensor) return built;
       cudaGetLastError();
-      packed = false;
-    } else if (dense(body, c.cells.bbox(0), h)) {
       packed = false;
     }
   }

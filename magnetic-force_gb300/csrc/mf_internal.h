@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <string>
+#include <functional>
 #include <vector>
 
 #include "../../include/mf.h"
@@ -395,8 +396,10 @@ class CellList {
   // Bins the particles of every scene into cells of edge >= 2h; particles of
   // a cell are listed in increasing index order (deterministic sums).
   // Synchronises `st` once (the bounding boxes are read on the host).
+  // wanted (optional) gets a scene's bounding box before anything is binned;
+  // where it says no the list is left unbuilt, not to be used.
   mf_status build(const float4* pos4, const std::vector<CellSceneSpec>& scenes, cudaStream_t st,
-                  double margin_h = 0.0);
+                  double margin_h = 0.0, const std::function<bool(const double*)>& wanted = {});
   // Re-bins moved particles on the grids of the last build (no host
   // synchronisation, so it can be captured in a CUDA graph).  Particles that
   // left a grid are binned into its border cells, which keeps every
